@@ -1,147 +1,306 @@
 // Device-side BCSR construction.
 //
-//   CSR -> BCSR: the layout contract of csr_to_bcsr_cpu (core/wrapper/convert_wrapper.cpp:27-180),
-//   built with one stable radix sort instead of per-window std::sort on the host: every edge
-//   gets the key (window, column, row-in-window); sorted, equal (window, column) runs become one
-//   column slot, slot / 8 is the tile, and the last duplicate of a (row, column) pair wins
-//   (convert_wrapper.cpp:174).
+//   CSR -> BCSR: the layout contract of csr_to_bcsr_cpu (core/wrapper/convert_wrapper.cpp:27-180).
+//   The entries of a 16-row window are one contiguous range of the CSR arrays, so a window is
+//   built by itself: its entries are ordered by (column, row), equal columns become one column
+//   slot, slot / 8 is the tile, and the last duplicate of a (row, column) pair wins
+//   (convert_wrapper.cpp:174).  No pass goes over the whole graph more than once per phase.
 //
 //   BCSR -> transposed CSR: extracts the non-zero entries of the tiles as (column, row, value)
 //   so that the transposed adjacency can be built once, cached and multiplied with the forward
 //   kernel; this replaces the per-call atomic scatter of spmm_bcsr_transpose_atomic_kernel
 //   (core/include/spmm_tc.cuh:211-270).
 //
-// cub::DeviceRadixSort / DeviceScan (CUDA toolkit) do the sort and the prefix sums; this is
-// graph preparation, not the per-step hot loop.
+// cub::DeviceScan (CUDA toolkit) does the prefix sums over windows and columns.
 #include <cub/cub.cuh>
 
 #include "grws_common.cuh"
 
 namespace grws {
 
-constexpr int ROW_BITS = 4;   // row inside a 16-row window
-// Key of an entry that does not exist (a padding slot of a fixed-stride neighbour list, the unused
-// tail of a CSR array sized by a bound).  Real keys are below it (fewer than 2^28 windows), so such
-// entries sort to the end; they open no column slot and write nothing.
-constexpr uint64_t INVALID_KEY = ~0ull;
+// A window of up to SMALL_ENTRIES entries is sorted by one warp in registers (16 keys a lane); a larger
+// one is ranked by a CTA through a bitmap of its columns, whose cost does not grow with log(entries).
+// 512 covers every block of a sampled step up to fan-out 32 and all but the hub windows of a power-law
+// graph; 32 keys a lane would spill.
+constexpr int SMALL_ENTRIES = 512;
+constexpr int COUNT_WARPS = 8;
+constexpr int LARGE_THREADS = 1024;
+constexpr int BITMAP_WORDS = 16384;                // 524,288 columns per round of a large window
+constexpr int LARGE_SMEM = BITMAP_WORDS * 4 + BITMAP_WORDS / 2 * 4;   // bits + one prefix per word pair: two CTAs per SM
+constexpr int FILL_WARPS = 8;
+constexpr int FILL_BYTES = 4096;                   // tiles a warp assembles in shared memory at a time
+constexpr int FILL_LARGE_THREADS = 512;            // one warp per row of a window
 
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
-// layout of the scratch buffer shared by the count and fill phases of csr_to_bcsr
+// The entries of a matrix by rows: a CSR (row_ptr set), or fixed-stride lists of `fanout` slots per row
+// whose empty slots hold a negative id.
+struct EntrySource {
+    const int64_t *row_ptr;
+    const int32_t *col;
+    const float *val;
+    int64_t num_rows;
+    int fanout;
+    __device__ __forceinline__ int64_t row_start(int64_t r) const {
+        r = r < num_rows ? r : num_rows;
+        return row_ptr ? row_ptr[r] : r * fanout;
+    }
+    // lists: a negative id is an empty slot; CSR ids are taken as they are (ordered as unsigned)
+    __device__ __forceinline__ bool empty(int32_t c) const { return row_ptr == nullptr && c < 0; }
+};
+
+// Scratch shared by the count and fill phases.
+//   rec, of a window of at most SMALL_ENTRIES entries (ordered by column slot):
+//         column << 32 | slot << 5 | row in window << 1 | 1 if the entry is not written (an empty list
+//         slot, or an earlier duplicate of the same row and column)
+//   rec, of a larger window (in the order of the source): column << 32 | slot, all ones for an empty slot
 struct BuildScratch {
-    uint64_t *keys_a, *keys_b;
-    float *vals_a, *vals_b;
-    int32_t *flags;         // per sorted entry: 1 when it opens a new (window, column) run
-    int32_t *uidx;          // per sorted entry: 1 + global index of its (window, column) slot (inclusive scan of flags)
-    int32_t *nuniq;         // [W+2] unique columns per window
-    int32_t *ufirst;        // [W+2] exclusive scan of nuniq
-    int64_t *tiles;         // [W+2] tiles per window, shifted by one
-    int32_t *col_bits;      // bits of the column field of the keys (the count phase leaves it for the fill phase)
+    uint64_t *rec;
+    float *val;             // value of the entry rec describes
+    int32_t *row_start;     // [num_rows + 1]
+    int64_t *tiles;         // [W+1] tiles per window, shifted by one
+    int32_t *large;         // [1 + W] number of large windows, then their ids in no fixed order
     void *cub_tmp;
     size_t cub_bytes;
     size_t total;
 };
 
-static size_t cub_temp_bytes(int64_t nnz, int64_t W) {
-    size_t s1 = 0, s2 = 0, s3 = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, s1, (const uint64_t *)nullptr, (uint64_t *)nullptr,
-                                    (const float *)nullptr, (float *)nullptr, (int)nnz, 0, 64);
-    cub::DeviceScan::InclusiveSum(nullptr, s2, (const int32_t *)nullptr, (int32_t *)nullptr, (int)nnz);
-    cub::DeviceScan::InclusiveSum(nullptr, s3, (const int64_t *)nullptr, (int64_t *)nullptr, (int)(W + 1));
-    size_t m = s1 > s2 ? s1 : s2;
-    return m > s3 ? m : s3;
+static size_t scan_temp_bytes(int64_t n) {
+    size_t s = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, s, (const int64_t *)nullptr, (int64_t *)nullptr, (int)n);
+    return s;
 }
 
-static BuildScratch carve(void *base, int64_t nnz, int64_t W) {
+static BuildScratch carve(void *base, int64_t nnz, int64_t num_rows) {
     BuildScratch s;
+    const int64_t W = ceil_div(num_rows, TILE_ROWS);
     char *p = static_cast<char *>(base);
     size_t off = 0;
     auto take = [&](size_t bytes) { char *q = p ? p + off : nullptr; off += align_up(bytes); return (void *)q; };
     const size_t n = (size_t)(nnz > 0 ? nnz : 1);
-    s.keys_a = (uint64_t *)take(n * 8);
-    s.keys_b = (uint64_t *)take(n * 8);
-    s.vals_a = (float *)take(n * 4);
-    s.vals_b = (float *)take(n * 4);
-    s.flags = (int32_t *)take(n * 4);
-    s.uidx = (int32_t *)take(n * 4);
-    s.nuniq = (int32_t *)take((size_t)(W + 2) * 4);
-    s.ufirst = (int32_t *)take((size_t)(W + 2) * 4);
-    s.tiles = (int64_t *)take((size_t)(W + 2) * 8);
-    s.col_bits = (int32_t *)take(64);
-    s.cub_bytes = cub_temp_bytes(nnz, W);
+    s.rec = (uint64_t *)take(n * 8);
+    s.val = (float *)take(n * 4);
+    s.row_start = (int32_t *)take((size_t)(num_rows + 1) * 4);
+    s.tiles = (int64_t *)take((size_t)(W + 1) * 8);
+    s.large = (int32_t *)take((size_t)(W + 1) * 4);
+    s.cub_bytes = scan_temp_bytes(W + 1);
     s.cub_tmp = take(s.cub_bytes);
     s.total = off;
     return s;
 }
 
-// Sort key of an entry: window | column | row-in-window.  The column field has as many bits as the
-// caller's bound on the column ids needs (32 without a bound), so that the radix sort, which runs one
-// pass per 8 key bits, has fewer passes to make: the blocks of a sampled step have 2^13 windows and 2^21
-// columns at most, 38 key bits instead of 49.  A column field of b bits holds ids below 2^b - 1 only,
-// which keeps the invalid key (all ones) apart from every real key within the sorted bits.
-__host__ __device__ __forceinline__ uint64_t make_key(int64_t row, int32_t col, int col_bits) {
-    return ((uint64_t)(row / TILE_ROWS) << (col_bits + ROW_BITS)) | ((uint64_t)(uint32_t)col << ROW_BITS) | (uint64_t)(row % TILE_ROWS);
-}
-
-static int column_bits(int64_t num_cols_bound) {
-    if (num_cols_bound <= 0 || num_cols_bound >= (1LL << 31)) return 32;
-    int b = 0;
-    for (int64_t x = num_cols_bound; x > 0; x >>= 1) ++b;      // ids < bound <= 2^b - 1
-    return b;
-}
-
-__global__ void make_keys_kernel(int64_t num_rows, const int64_t *__restrict__ row_ptr,
-                                 const int32_t *__restrict__ col_idx, uint64_t *__restrict__ keys, int col_bits) {
-    // one warp per row
-    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (row >= num_rows) return;
-    const int64_t e0 = row_ptr[row], e1 = row_ptr[row + 1];
-    for (int64_t e = e0 + lane; e < e1; e += 32)
-        keys[e] = make_key(row, col_idx[e], col_bits);
-}
-
-// keys of a hop's fixed-stride neighbour lists: entry (row i, slot j) holds local column id
-// local[i * fanout + j], or -1 when the slot is empty
-__global__ void make_keys_lists_kernel(int64_t n_entries, int fanout, const int32_t *__restrict__ local,
-                                       uint64_t *__restrict__ keys, int col_bits) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_entries) return;
-    const int32_t c = local[e];
-    const int64_t row = e / fanout;
-    keys[e] = c < 0 ? INVALID_KEY : make_key(row, c, col_bits);
-}
-
-__global__ void head_flags_kernel(int64_t nnz, const uint64_t *__restrict__ keys,
-                                  int32_t *__restrict__ flags, int32_t *__restrict__ nuniq, int col_bits,
-                                  int32_t *__restrict__ col_bits_out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool head = false;
-    uint64_t window = 0;
-    if (i < nnz) {
-        if (i == 0) *col_bits_out = col_bits;              // the fill phase decodes the keys with it
-        const uint64_t key = keys[i];
-        if (key != INVALID_KEY) {
-            const uint64_t k = key >> ROW_BITS;
-            head = (i == 0) || ((keys[i - 1] >> ROW_BITS) != k);
-            window = k >> col_bits;
+// Ascending bitonic sort of 32 * E keys held by one warp; key i is k[i % E] of lane i / E.
+template <int E>
+__device__ __forceinline__ void warp_sort(uint64_t (&k)[E], int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32 * E; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= E) {
+                const int ls = stride / E;
+                const bool up = (lane & (size / E)) == 0;            // size == 32 * E: every lane's bit is 0
+                const bool keep_min = ((lane & ls) == 0) == up;
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const uint64_t o = __shfl_xor_sync(0xffffffffu, k[e], ls);
+                    k[e] = (k[e] < o) == keep_min ? k[e] : o;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    if (e & stride) continue;
+                    const bool up = size < E ? (e & size) == 0 : (lane & (size / E)) == 0;
+                    const uint64_t a = k[e], b = k[e + stride];
+                    const bool swap = (a > b) == up;
+                    k[e] = swap ? b : a;
+                    k[e + stride] = swap ? a : b;
+                }
+            }
         }
-        flags[i] = head ? 1 : 0;
-    }
-    // The keys are sorted, so the heads a warp sees belong to one or two windows almost always: one
-    // atomic per window and warp instead of one per head (a window's counter otherwise takes
-    // hundreds of atomics from neighbouring threads).
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    if (head) {
-        const unsigned same = __match_any_sync(heads, window);
-        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(nuniq + window, __popc(same));
     }
 }
 
-__global__ void tiles_kernel(int64_t W, const int32_t *__restrict__ nuniq, int64_t *__restrict__ tiles) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w > W) return;
-    tiles[w] = (w == 0) ? 0 : (nuniq[w - 1] + TILE_COLS - 1) / TILE_COLS;   // shifted by one for an inclusive scan
+// Sorts one window's `m` entries, gives every distinct column its slot and writes the records in
+// order.  `ends`: in lanes 0..15, where the entries of that row end, counted from the window's first.
+template <int E>
+__device__ __forceinline__ int sort_window(const EntrySource &src, int64_t s, int m, int ends, int lane,
+                                           uint64_t *__restrict__ rec, float *__restrict__ val) {
+    constexpr uint64_t NONE = ~0ull;
+    uint64_t k[E];                                                    // column 32 | row 4 | position 12
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int p = e * 32 + lane;
+        const int32_t c = p < m ? __ldg(src.col + s + p) : 0;
+        int row = 0;
+#pragma unroll
+        for (int step = TILE_ROWS / 2; step > 0; step >>= 1)          // number of rows that end at or before p
+            row += p >= __shfl_sync(0xffffffffu, ends, row + step - 1) ? step : 0;
+        k[e] = p < m && !src.empty(c) ? (uint64_t)(uint32_t)c << 16 | (uint64_t)(row << 12 | p) : NONE;
+    }
+    warp_sort<E>(k, lane);
+    const uint64_t before = __shfl_up_sync(0xffffffffu, k[E - 1], 1), after = __shfl_down_sync(0xffffffffu, k[0], 1);
+    int heads = 0;
+    bool head[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const bool first = e == 0 && lane == 0;
+        const uint64_t prev = e == 0 ? before : k[e > 0 ? e - 1 : 0];
+        head[e] = k[e] != NONE && (first || (prev >> 16) != (k[e] >> 16));
+        heads += head[e];
+    }
+    int incl = heads;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    int slot = incl - heads - 1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = lane * E + e;
+        slot += head[e];
+        if (i >= m) continue;
+        const bool last = e == E - 1 && lane == 31;
+        const uint64_t next = last ? NONE : (e == E - 1 ? after : k[e < E - 1 ? e + 1 : 0]);
+        const bool drop = k[e] == NONE || (next != NONE && (next >> 12) == (k[e] >> 12));
+        const uint32_t col = (uint32_t)(k[e] >> 16), row = (uint32_t)(k[e] >> 12) & (TILE_ROWS - 1);
+        rec[s + i] = (uint64_t)col << 32 | (uint64_t)((uint32_t)slot << 5 | row << 1 | (drop ? 1u : 0u));
+        val[s + i] = drop ? 0.f : __ldg(src.val + s + (int)(k[e] & 0xfff));
+    }
+    return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// One warp per window.  Bound by instruction issue (the compare-exchange network: 36 steps of 8 keys a lane
+// for the usual window of up to 256 entries).  Against one radix sort of 64-bit (window, column, row) keys over all
+// entries -- five to seven passes over keys and values, flags, two scans -- a mini-batch of 1,024 seeds and
+// fan-out 15-10-5 is sampled and built in 519 us instead of 769.
+__global__ void __launch_bounds__(COUNT_WARPS * 32)
+count_windows_kernel(const EntrySource src, int64_t W, BuildScratch s) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)blockIdx.x * COUNT_WARPS + (threadIdx.x >> 5);
+    if (w >= W) return;
+    const int64_t r0 = w * TILE_ROWS, row = r0 + lane;
+    const int64_t end = src.row_start(row + 1);                       // rows past the last one are empty
+    const int64_t first = __shfl_sync(0xffffffffu, src.row_start(r0), 0);
+    const int64_t total = __shfl_sync(0xffffffffu, end, TILE_ROWS - 1) - first;
+    if (lane < TILE_ROWS && row < src.num_rows) s.row_start[row + 1] = (int32_t)end;
+    if (w == 0 && lane == 0) { s.row_start[0] = (int32_t)first; s.tiles[0] = 0; }
+    if (total > SMALL_ENTRIES) {
+        if (lane == 0) s.large[1 + atomicAdd(s.large, 1)] = (int32_t)w;
+        return;
+    }
+    const int m = (int)total, ends = (int)(end - first);
+    int n = 0;
+    if (m > 256) n = sort_window<16>(src, first, m, ends, lane, s.rec, s.val);
+    else if (m > 128) n = sort_window<8>(src, first, m, ends, lane, s.rec, s.val);
+    else if (m > 64) n = sort_window<4>(src, first, m, ends, lane, s.rec, s.val);
+    else if (m > 32) n = sort_window<2>(src, first, m, ends, lane, s.rec, s.val);
+    else if (m > 0) n = sort_window<1>(src, first, m, ends, lane, s.rec, s.val);
+    if (lane == 0) s.tiles[w + 1] = (n + TILE_COLS - 1) / TILE_COLS;
+}
+
+__device__ __forceinline__ uint32_t block_reduce(uint32_t v, bool take_min, uint32_t *warp_part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = take_min ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+    __syncthreads();                                                  // the previous use of warp_part is over
+    if (lane == 0) warp_part[warp] = v;
+    __syncthreads();
+    v = warp_part[lane];                                              // LARGE_THREADS / 32 == 32 warps
+    return take_min ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+}
+
+// Large windows, one CTA each: the columns that occur are marked in a bitmap in shared memory, a prefix sum
+// of its bit counts gives every column its slot.  A window whose columns span more than the bitmap takes
+// further rounds, each starting at the smallest column not yet numbered.
+__global__ void __launch_bounds__(LARGE_THREADS, 2)
+count_large_kernel(const EntrySource src, BuildScratch s) {
+    extern __shared__ uint32_t smem[];
+    __shared__ uint32_t warp_part[LARGE_THREADS / 32];
+    uint32_t *bits = smem, *prefix = smem + BITMAP_WORDS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_large = s.large[0];
+    for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
+        const int64_t w = s.large[1 + q], first = src.row_start(w * TILE_ROWS), m = src.row_start((w + 1) * TILE_ROWS) - first;
+        const int32_t *col = src.col + first;
+        uint32_t lo = 0xffffffffu, hi = 0;
+        bool any = false;
+        for (int64_t i = tid; i < m; i += LARGE_THREADS) {
+            const int32_t c = __ldg(col + i);
+            if (src.empty(c)) continue;
+            any = true;
+            lo = min(lo, (uint32_t)c);
+            hi = max(hi, (uint32_t)c);
+        }
+        any = __syncthreads_or(any);
+        lo = block_reduce(lo, true, warp_part);
+        hi = block_reduce(hi, false, warp_part);
+        uint32_t total = 0;
+        bool more = any;
+        while (more) {
+            const uint64_t left = (uint64_t)hi - lo + 1;
+            const uint32_t span = left < BITMAP_WORDS * 32ull ? (uint32_t)left : BITMAP_WORDS * 32u;
+            const int pairs = (int)((span + 63) / 64);
+            for (int i = tid; i < pairs; i += LARGE_THREADS) reinterpret_cast<uint2 *>(bits)[i] = make_uint2(0u, 0u);
+            __syncthreads();
+            uint32_t next = 0xffffffffu;
+            bool beyond = false;
+            for (int64_t i = tid; i < m; i += LARGE_THREADS) {
+                const int32_t c = __ldg(col + i);
+                if (src.empty(c) || (uint32_t)c < lo) continue;
+                const uint32_t x = (uint32_t)c - lo;
+                if (x < span) {
+                    atomicOr(bits + (x >> 5), 1u << (x & 31));
+                } else {
+                    beyond = true;
+                    next = min(next, (uint32_t)c);
+                }
+            }
+            more = __syncthreads_or(beyond);
+            // exclusive prefix of the bit counts, one word pair at a time per thread
+            const int each = (pairs + LARGE_THREADS - 1) / LARGE_THREADS, p0 = tid * each, p1 = min(pairs, p0 + each);
+            uint32_t sum = 0;
+            for (int i = p0; i < p1; ++i) {
+                const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
+                sum += __popc(v.x) + __popc(v.y);
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            if (lane == 31) warp_part[warp] = incl;
+            __syncthreads();
+            const uint32_t part = warp_part[lane];
+            const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? part : 0u);
+            const uint32_t round = __reduce_add_sync(0xffffffffu, part);
+            uint32_t at = total + ahead + incl - sum;
+            for (int i = p0; i < p1; ++i) {
+                const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
+                prefix[i] = at;
+                at += __popc(v.x) + __popc(v.y);
+            }
+            __syncthreads();
+            for (int64_t i = tid; i < m; i += LARGE_THREADS) {
+                const int32_t c = __ldg(col + i);
+                if (src.empty(c) || (uint32_t)c < lo) continue;
+                const uint32_t x = (uint32_t)c - lo;
+                if (x >= span) continue;
+                const uint2 v = reinterpret_cast<uint2 *>(bits)[x >> 6];
+                const uint32_t below = (1u << (x & 31)) - 1u;
+                const uint32_t slot = prefix[x >> 6] + (x & 32 ? __popc(v.x) + __popc(v.y & below) : __popc(v.x & below));
+                s.rec[first + i] = (uint64_t)(uint32_t)c << 32 | slot;
+            }
+            total += round;
+            if (more) lo = block_reduce(next, true, warp_part);
+            __syncthreads();                                          // bits and prefix are free again
+        }
+        for (int64_t i = tid; i < m; i += LARGE_THREADS) {
+            if (src.empty(__ldg(col + i))) s.rec[first + i] = ~0ull;
+            s.val[first + i] = __ldg(src.val + first + i);
+        }
+        if (tid == 0) s.tiles[w + 1] = ((int64_t)total + TILE_COLS - 1) / TILE_COLS;
+    }
 }
 
 template <typename T> __device__ __forceinline__ T from_float(float v);
@@ -149,29 +308,110 @@ template <> __device__ __forceinline__ float from_float<float>(float v) { return
 template <> __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
+// 16 bytes of an output array at piece index i; an array that does not start on a 16-byte boundary takes
+// them element by element
 template <typename T>
-__global__ void fill_kernel(int64_t nnz, const uint64_t *__restrict__ keys, const float *__restrict__ vals,
-                            const int32_t *__restrict__ uidx, const int32_t *__restrict__ ufirst,
-                            const int64_t *__restrict__ window_offset, int32_t *__restrict__ out_cols,
-                            T *__restrict__ out_vals, const int32_t *__restrict__ col_bits_in) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    const uint64_t key = keys[i];
-    if (key == INVALID_KEY) return;
-    if (i + 1 < nnz && keys[i + 1] == key) return;          // an identical (row, column) follows: it wins
-    const int col_bits = *col_bits_in;
-    const int64_t w = (int64_t)(key >> (col_bits + ROW_BITS));
-    const int32_t col = (int32_t)((key >> ROW_BITS) & ((1ull << col_bits) - 1ull));
-    const int r = (int)(key & (TILE_ROWS - 1));
-    const int32_t slot = uidx[i] - 1 - ufirst[w];
-    const int64_t tile = window_offset[w] + slot / TILE_COLS;
-    const int ic = slot % TILE_COLS;
-    out_cols[tile * TILE_COLS + ic] = col;                    // every entry of the run writes the same id
-    out_vals[tile * TILE_ELEMS + r * TILE_COLS + ic] = from_float<T>(vals[i]);
+__device__ __forceinline__ void store_piece(T *p, int64_t i, uint4 v, bool vec) {
+    if (vec) {
+        reinterpret_cast<uint4 *>(p)[i] = v;
+    } else {
+        const T *e = reinterpret_cast<const T *>(&v);
+#pragma unroll
+        for (int j = 0; j < 16 / (int)sizeof(T); ++j) p[i * (16 / (int)sizeof(T)) + j] = e[j];
+    }
 }
 
-__global__ void fill_i32_kernel(int32_t *p, int64_t n, int32_t v) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
+// One warp per window: the records are in slot order, so a group of consecutive tiles is a run of them; it is
+// assembled in shared memory and written once, in 16-byte pieces.  Bound by the bytes of the tiles.
+// All threads then empty the tiles behind the last one (arrays sized by a bound).
+template <typename T>
+__global__ void __launch_bounds__(FILL_WARPS * 32)
+fill_windows_kernel(int64_t W, int64_t num_rows, int64_t num_tiles, const BuildScratch s, const int64_t *__restrict__ window_offset,
+                    int32_t *__restrict__ out_cols, T *__restrict__ out_vals, bool vec) {
+    constexpr int GROUP = FILL_BYTES / (TILE_ELEMS * (int)sizeof(T));           // tiles per group
+    constexpr int TILE_V = TILE_ELEMS * (int)sizeof(T) / 16;                    // 16-byte pieces of a tile
+    __shared__ __align__(16) T tile_buf[FILL_WARPS][GROUP * TILE_ELEMS];
+    __shared__ __align__(16) int32_t col_buf[FILL_WARPS][GROUP * TILE_COLS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t w = (int64_t)blockIdx.x * FILL_WARPS + warp;
+    if (w < W) {
+        const int64_t t0 = window_offset[w], nt = window_offset[w + 1] - t0;
+        const int64_t r1 = (w + 1) * TILE_ROWS < num_rows ? (w + 1) * TILE_ROWS : num_rows;
+        int p = s.row_start[w * TILE_ROWS];
+        const int end = s.row_start[r1];
+        if (end - p <= SMALL_ENTRIES) {
+            T *tb = tile_buf[warp];
+            int32_t *cb = col_buf[warp];
+            for (int g = 0; g < nt; g += GROUP) {
+#pragma unroll
+                for (int i = 0; i < FILL_BYTES / 512; ++i) reinterpret_cast<uint4 *>(tb)[i * 32 + lane] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int i = 0; i < GROUP * TILE_COLS / 32; ++i) cb[i * 32 + lane] = -1;
+                __syncwarp();
+                while (p < end) {
+                    const int q = p + lane;
+                    const uint64_t r = q < end ? __ldg(s.rec + q) : ~0ull;
+                    const float v = q < end ? __ldg(s.val + q) : 0.f;
+                    const uint32_t info = (uint32_t)r;
+                    const int slot = (int)(info >> 5) - g * TILE_COLS;
+                    const bool in = q < end && slot < GROUP * TILE_COLS;
+                    if (in && !(info & 1u)) {
+                        tb[(slot >> 3) * TILE_ELEMS + ((info >> 1) & (TILE_ROWS - 1)) * TILE_COLS + (slot & 7)] = from_float<T>(v);
+                        cb[slot] = (int32_t)(r >> 32);
+                    }
+                    const int n = __popc(__ballot_sync(0xffffffffu, in));
+                    p += n;
+                    if (n < 32) break;
+                }
+                __syncwarp();
+                const int live = nt - g < GROUP ? (int)(nt - g) : GROUP;
+                T *ov = out_vals + (t0 + g) * TILE_ELEMS;
+                int32_t *oc = out_cols + (t0 + g) * TILE_COLS;
+                for (int i = lane; i < live * TILE_V; i += 32) store_piece(ov, i, reinterpret_cast<uint4 *>(tb)[i], vec);
+                for (int i = lane; i < live * 2; i += 32) store_piece(oc, i, reinterpret_cast<uint4 *>(cb)[i], vec);
+                __syncwarp();
+            }
+        }
+    }
+    const int64_t T0 = window_offset[W], stride = (int64_t)gridDim.x * blockDim.x, me = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t i = T0 * TILE_V + me; i < num_tiles * TILE_V; i += stride) store_piece(out_vals, i, make_uint4(0u, 0u, 0u, 0u), vec);
+    for (int64_t i = T0 * 2 + me; i < num_tiles * 2; i += stride)
+        store_piece(out_cols, i, make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), vec);
+}
+
+// Large windows, one CTA each: empty tiles, then a warp per row scatters that row's entries in their order,
+// so that the last of several entries of one column is the one that stays.
+template <typename T>
+__global__ void __launch_bounds__(FILL_LARGE_THREADS)
+fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restrict__ window_offset,
+                  int32_t *__restrict__ out_cols, T *__restrict__ out_vals, bool vec) {
+    constexpr int TILE_V = TILE_ELEMS * (int)sizeof(T) / 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_large = s.large[0];
+    for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
+        const int64_t w = s.large[1 + q], t0 = window_offset[w], nt = window_offset[w + 1] - t0;
+        T *ov = out_vals + t0 * TILE_ELEMS;
+        int32_t *oc = out_cols + t0 * TILE_COLS;
+        for (int64_t i = threadIdx.x; i < nt * TILE_V; i += FILL_LARGE_THREADS) store_piece(ov, i, make_uint4(0u, 0u, 0u, 0u), vec);
+        for (int64_t i = threadIdx.x; i < nt * 2; i += FILL_LARGE_THREADS)
+            store_piece(oc, i, make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), vec);
+        __syncthreads();
+        const int64_t row = w * TILE_ROWS + warp;
+        if (row < num_rows) {
+            const int64_t end = s.row_start[row + 1];
+            for (int64_t b = s.row_start[row]; b < end; b += 32) {
+                const uint64_t r = b + lane < end ? __ldg(s.rec + b + lane) : ~0ull;
+                const float v = b + lane < end ? __ldg(s.val + b + lane) : 0.f;
+                const uint32_t slot = (uint32_t)r;
+                const unsigned same = __match_any_sync(0xffffffffu, r);
+                if (r != ~0ull && lane == 31 - __clz(same)) {
+                    ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v);
+                    oc[slot] = (int32_t)(r >> 32);
+                }
+                __syncwarp();
+            }
+        }
+    }
 }
 
 static inline unsigned blocks_for(int64_t n, int threads) {
@@ -242,34 +482,52 @@ __global__ void bcsr_rows_kernel(int64_t W, int64_t num_rows, const int64_t *__r
     if (MODE == 0) row_ptr[row + 1] = o;
 }
 
+int block_build_fill(int64_t n_dst, int fanout, const int64_t *window_offset, int64_t num_tiles, int32_t *out_cols, void *out_vals,
+                     int val_dtype, void *scratch, size_t scratch_bytes, cudaStream_t st);
+
 }  // namespace grws
 
 using namespace grws;
 
-// Second half of the count phase, shared by the CSR and the neighbour-list front ends: sorts the
-// keys in s.keys_a (values alongside), flags the first entry of every (window, column) run and
-// turns the unique-column counts into window_offset.
-static int count_from_keys(const BuildScratch &s, int64_t nnz, int64_t W, const float *values,
-                           int64_t *window_offset, int col_bits, cudaStream_t st) {
-    GRWS_CUDA_TRY(cudaMemsetAsync(s.nuniq, 0, (size_t)(W + 2) * 4, st));
-    if (nnz > 0) {
-        size_t tmp = s.cub_bytes;
-        // only the bits a key can use are sorted; the invalid key is all ones there too, so it
-        // still sorts behind every real key (no column id fills its field with ones)
-        int end_bit = col_bits + ROW_BITS;
-        for (int64_t x = W; x > 0; x >>= 1) ++end_bit;
-        if (end_bit > 64) end_bit = 64;
-        GRWS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(s.cub_tmp, tmp, s.keys_a, s.keys_b, values, s.vals_b,
-                                                      (int)nnz, 0, end_bit, st));
-        head_flags_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(nnz, s.keys_b, s.flags, s.nuniq, col_bits, s.col_bits);
-        tmp = s.cub_bytes;
-        GRWS_CUDA_TRY(cub::DeviceScan::InclusiveSum(s.cub_tmp, tmp, s.flags, s.uidx, (int)nnz, st));
+static int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        sms = 148;
+    return sms;
+}
+
+// Count phase of both front ends.  may_be_large: some window may have more than SMALL_ENTRIES entries.
+static int count_entries(const BuildScratch &s, const EntrySource &src, int64_t W, bool may_be_large, int64_t *window_offset,
+                         cudaStream_t st) {
+    if (W == 0) {
+        GRWS_CUDA_TRY(cudaMemsetAsync(window_offset, 0, 8, st));
+        return GRWS_OK;
     }
-    tiles_kernel<<<blocks_for(W + 1, 256), 256, 0, st>>>(W, s.nuniq, s.tiles);
+    GRWS_CUDA_TRY(cudaMemsetAsync(s.large, 0, 4, st));
+    count_windows_kernel<<<blocks_for(W, COUNT_WARPS), COUNT_WARPS * 32, 0, st>>>(src, W, s);
+    if (may_be_large) {
+        GRWS_CUDA_TRY(cudaFuncSetAttribute(count_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LARGE_SMEM));
+        const int64_t grid = 2 * sm_count();
+        count_large_kernel<<<(unsigned)(W < grid ? W : grid), LARGE_THREADS, LARGE_SMEM, st>>>(src, s);
+    }
     size_t tmp = s.cub_bytes;
     GRWS_CUDA_TRY(cub::DeviceScan::InclusiveSum(s.cub_tmp, tmp, s.tiles, window_offset, (int)(W + 1), st));
-    tmp = s.cub_bytes;
-    GRWS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(s.cub_tmp, tmp, s.nuniq, s.ufirst, (int)(W + 1), st));
+    GRWS_CUDA_TRY(cudaGetLastError());
+    return GRWS_OK;
+}
+
+template <typename T>
+static int fill_entries(const BuildScratch &s, int64_t num_rows, int64_t num_tiles, bool may_be_large, const int64_t *window_offset,
+                        int32_t *out_cols, void *out_vals, cudaStream_t st) {
+    const int64_t W = ceil_div(num_rows, TILE_ROWS);
+    const bool vec = aligned16(out_cols) && aligned16(out_vals);
+    fill_windows_kernel<T><<<blocks_for(W, FILL_WARPS), FILL_WARPS * 32, 0, st>>>(W, num_rows, num_tiles, s, window_offset, out_cols,
+                                                                                  static_cast<T *>(out_vals), vec);
+    if (may_be_large) {
+        const int64_t grid = 4 * sm_count();
+        fill_large_kernel<T><<<(unsigned)(W < grid ? W : grid), FILL_LARGE_THREADS, 0, st>>>(num_rows, s, window_offset, out_cols,
+                                                                                            static_cast<T *>(out_vals), vec);
+    }
     GRWS_CUDA_TRY(cudaGetLastError());
     return GRWS_OK;
 }
@@ -290,49 +548,62 @@ static int transpose_count(const int64_t *wo, const int32_t *cols, const void *v
 }
 
 
+// a window of fixed-stride lists has 16 * fanout slots
+static bool lists_may_be_large(int fanout) { return (int64_t)fanout * TILE_ROWS > SMALL_ENTRIES; }
+
+static int fill_any(int64_t num_rows, int64_t nnz, bool may_be_large, const int64_t *window_offset, int64_t num_tiles, int32_t *out_cols,
+                    void *out_vals, int val_dtype, void *scratch, size_t scratch_bytes, cudaStream_t st) {
+    GRWS_REQUIRE(num_rows >= 0 && nnz >= 0 && num_tiles >= 0, "negative size");
+    BuildScratch s = carve(scratch, nnz, num_rows);
+    if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small");
+    if (num_tiles == 0) return GRWS_OK;
+    GRWS_REQUIRE(window_offset && out_cols && out_vals && scratch, "null pointer");
+    switch (val_dtype) {
+        case GRWS_F32: return fill_entries<float>(s, num_rows, num_tiles, may_be_large, window_offset, out_cols, out_vals, st);
+        case GRWS_F16: return fill_entries<__half>(s, num_rows, num_tiles, may_be_large, window_offset, out_cols, out_vals, st);
+        case GRWS_BF16: return fill_entries<__nv_bfloat16>(s, num_rows, num_tiles, may_be_large, window_offset, out_cols, out_vals, st);
+    }
+    return fail(GRWS_ERR_UNSUPPORTED, "bad value dtype %d", val_dtype);
+}
+
+// the fill phase of a block built from lists (sampler.cu): the host knows how large its windows can be
+int grws::block_build_fill(int64_t n_dst, int fanout, const int64_t *window_offset, int64_t num_tiles, int32_t *out_cols, void *out_vals,
+                           int val_dtype, void *scratch, size_t scratch_bytes, cudaStream_t st) {
+    return fill_any(n_dst, n_dst * fanout, lists_may_be_large(fanout), window_offset, num_tiles, out_cols, out_vals, val_dtype, scratch,
+                    scratch_bytes, st);
+}
+
 extern "C" {
 
 __attribute__((visibility("default")))
 size_t grws_csr_to_bcsr_scratch_bytes(int64_t num_rows, int64_t nnz) {
     if (num_rows < 0 || nnz < 0) return 0;
-    return carve(nullptr, nnz, ceil_div(num_rows, TILE_ROWS)).total;
-}
-
-static int csr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx, const float *values,
-                     int64_t nnz, bool nnz_is_bound, int64_t num_cols_bound, int64_t *window_offset, void *scratch,
-                     size_t scratch_bytes, void *stream) {
-    GRWS_REQUIRE(num_rows >= 0 && nnz >= 0, "negative size");
-    GRWS_REQUIRE(nnz < 0x7fffffffLL, "csr_to_bcsr handles fewer than 2^31 entries");
-    const int64_t W = ceil_div(num_rows, TILE_ROWS);
-    GRWS_REQUIRE(W < (1LL << 28), "too many windows");
-    GRWS_REQUIRE(row_ptr && window_offset && scratch, "null pointer");
-    GRWS_REQUIRE(nnz == 0 || (col_idx && values), "null CSR arrays");
-    BuildScratch s = carve(scratch, nnz, W);
-    if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small: %zu < %zu", scratch_bytes, s.total);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int col_bits = column_bits(num_cols_bound);
-    if (nnz > 0) {
-        // entries of the arrays past row_ptr[num_rows] (a CSR sized by a bound) keep the invalid key
-        if (nnz_is_bound) GRWS_CUDA_TRY(cudaMemsetAsync(s.keys_a, 0xff, (size_t)nnz * 8, st));
-        make_keys_kernel<<<blocks_for(num_rows * 32, 256), 256, 0, st>>>(num_rows, row_ptr, col_idx, s.keys_a, col_bits);
-    }
-    return count_from_keys(s, nnz, W, values, window_offset, col_bits, st);
+    return carve(nullptr, nnz, num_rows).total;
 }
 
 __attribute__((visibility("default")))
 int grws_csr_to_bcsr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
                            const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
                            size_t scratch_bytes, void *stream) {
-    return csr_count(num_rows, row_ptr, col_idx, values, nnz, false, 0, window_offset, scratch, scratch_bytes, stream);
+    GRWS_REQUIRE(num_rows >= 0 && nnz >= 0, "negative size");
+    GRWS_REQUIRE(nnz < 0x7fffffffLL, "csr_to_bcsr handles fewer than 2^31 entries");
+    const int64_t W = ceil_div(num_rows, TILE_ROWS);
+    GRWS_REQUIRE(W < (1LL << 28), "too many windows");
+    GRWS_REQUIRE(row_ptr && window_offset && scratch, "null pointer");
+    GRWS_REQUIRE(nnz == 0 || (col_idx && values), "null CSR arrays");
+    BuildScratch s = carve(scratch, nnz, num_rows);
+    if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small: %zu < %zu", scratch_bytes, s.total);
+    const EntrySource src = {row_ptr, col_idx, values, num_rows, 0};
+    return count_entries(s, src, W, nnz > SMALL_ENTRIES, window_offset, static_cast<cudaStream_t>(stream));
 }
 
+// The kernels only visit the entries that row_ptr covers, so a bound on their number needs nothing of its own.
 __attribute__((visibility("default")))
 int grws_csr_to_bcsr_count_bounded(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
                                    const float *values, int64_t nnz_bound, int64_t num_cols_bound,
                                    int64_t *window_offset, void *scratch, size_t scratch_bytes, void *stream) {
     GRWS_REQUIRE(num_cols_bound >= 0, "negative size");
-    return csr_count(num_rows, row_ptr, col_idx, values, nnz_bound, true, num_cols_bound, window_offset, scratch, scratch_bytes,
-                     stream);
+    return grws_csr_to_bcsr_count(num_rows, row_ptr, col_idx, values, nnz_bound, window_offset, scratch, scratch_bytes, stream);
 }
 
 __attribute__((visibility("default")))
@@ -343,42 +614,18 @@ int grws_block_build_count(const int32_t *local, const float *w, int64_t n_dst, 
     GRWS_REQUIRE(n_entries < 0x7fffffffLL, "hop too large");
     const int64_t W = ceil_div(n_dst, TILE_ROWS);
     GRWS_REQUIRE(window_offset && scratch && (n_entries == 0 || (local && w)), "null pointer");
-    BuildScratch s = carve(scratch, n_entries, W);
+    BuildScratch s = carve(scratch, n_entries, n_dst);
     if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "block build scratch too small: %zu < %zu", scratch_bytes, s.total);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int col_bits = column_bits(num_cols_bound);
-    if (n_entries > 0)
-        make_keys_lists_kernel<<<blocks_for(n_entries, 256), 256, 0, st>>>(n_entries, fanout, local, s.keys_a, col_bits);
-    return count_from_keys(s, n_entries, W, w, window_offset, col_bits, st);
+    const EntrySource src = {nullptr, local, w, n_dst, fanout};
+    return count_entries(s, src, W, lists_may_be_large(fanout), window_offset, static_cast<cudaStream_t>(stream));
 }
 
 __attribute__((visibility("default")))
 int grws_csr_to_bcsr_fill(int64_t num_rows, int64_t nnz, const int64_t *window_offset, int64_t num_tiles,
                           int32_t *out_cols, void *out_vals, int val_dtype, void *scratch,
                           size_t scratch_bytes, void *stream) {
-    GRWS_REQUIRE(num_rows >= 0 && nnz >= 0 && num_tiles >= 0, "negative size");
-    const int64_t W = ceil_div(num_rows, TILE_ROWS);
-    BuildScratch s = carve(scratch, nnz, W);
-    if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small");
-    if (num_tiles == 0) return GRWS_OK;
-    GRWS_REQUIRE(window_offset && out_cols && out_vals && scratch, "null pointer");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const unsigned fill_blocks = blocks_for(num_tiles * TILE_COLS, 256);
-    fill_i32_kernel<<<fill_blocks > 4096 ? 4096 : fill_blocks, 256, 0, st>>>(out_cols, num_tiles * TILE_COLS, -1);
-    GRWS_CUDA_TRY(cudaMemsetAsync(out_vals, 0, (size_t)num_tiles * TILE_ELEMS * dtype_bytes(val_dtype), st));
-    if (nnz > 0) {
-        const unsigned nb = blocks_for(nnz, 256);
-        if (val_dtype == GRWS_F32)
-            fill_kernel<float><<<nb, 256, 0, st>>>(nnz, s.keys_b, s.vals_b, s.uidx, s.ufirst, window_offset, out_cols, (float *)out_vals, s.col_bits);
-        else if (val_dtype == GRWS_F16)
-            fill_kernel<__half><<<nb, 256, 0, st>>>(nnz, s.keys_b, s.vals_b, s.uidx, s.ufirst, window_offset, out_cols, (__half *)out_vals, s.col_bits);
-        else if (val_dtype == GRWS_BF16)
-            fill_kernel<__nv_bfloat16><<<nb, 256, 0, st>>>(nnz, s.keys_b, s.vals_b, s.uidx, s.ufirst, window_offset, out_cols, (__nv_bfloat16 *)out_vals, s.col_bits);
-        else
-            return fail(GRWS_ERR_UNSUPPORTED, "bad value dtype %d", val_dtype);
-    }
-    GRWS_CUDA_TRY(cudaGetLastError());
-    return GRWS_OK;
+    return fill_any(num_rows, nnz, nnz > SMALL_ENTRIES, window_offset, num_tiles, out_cols, out_vals, val_dtype, scratch, scratch_bytes,
+                    static_cast<cudaStream_t>(stream));
 }
 
 // counts[0] = 0, counts[c + 1] = non-zero entries in column c; then inclusive scan -> row_ptr of A^T

@@ -291,6 +291,10 @@ __global__ void hop_counts_kernel(const int32_t *__restrict__ n_new, const int32
     }
 }
 
+// bcsr_build.cu
+int block_build_fill(int64_t n_dst, int fanout, const int64_t *window_offset, int64_t num_tiles, int32_t *out_cols, void *out_vals,
+                     int val_dtype, void *scratch, size_t scratch_bytes, cudaStream_t st);
+
 static inline size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 static inline unsigned nblocks(int64_t n, int t) { int64_t b = (n + t - 1) / t; return (unsigned)(b < 1 ? 1 : b); }
 
@@ -444,9 +448,6 @@ int grws_sample_layers_sizes(int64_t num_seeds, const int *fanouts, int num_hops
 size_t grws_csr_to_bcsr_scratch_bytes(int64_t num_rows, int64_t nnz);
 int grws_block_build_count(const int32_t *local, const float *w, int64_t n_dst, int fanout, int64_t num_cols_bound,
                            int64_t *window_offset, void *scratch, size_t scratch_bytes, void *stream);
-int grws_csr_to_bcsr_fill(int64_t num_rows, int64_t nnz, const int64_t *window_offset, int64_t num_tiles,
-                          int32_t *out_cols, void *out_vals, int val_dtype, void *scratch, size_t scratch_bytes,
-                          void *stream);
 
 struct LayersScratch {
     int32_t *nbr, *local, *cnt;
@@ -532,8 +533,8 @@ int grws_sample_layers(const int64_t *row_ptr, const int32_t *col_idx, const flo
         localize_flat_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, d.keys, d.vals, mask, s.local);
         // 3. the hop's BCSR block straight from the fixed-stride lists
         if (int e = grws_block_build_count(s.local, s.w, nd, (int)f, n_src[h], out_window_offset[h], s.build, s.build_bytes, stream)) return e;
-        if (int e = grws_csr_to_bcsr_fill(nd, n_entries, out_window_offset[h], tiles[h], out_cols[h], out_vals[h], val_dtype,
-                                          s.build, s.build_bytes, stream)) return e;
+        if (int e = block_build_fill(nd, (int)f, out_window_offset[h], tiles[h], out_cols[h], out_vals[h], val_dtype, s.build,
+                                     s.build_bytes, st)) return e;
         if (out_counts)
             hop_counts_kernel<<<1, 1024, 0, st>>>(d.n_new, dst, nd, s.cnt, out_window_offset[h], W, out_counts + 4 * h);
         GRWS_CUDA_TRY(cudaGetLastError());

@@ -189,8 +189,7 @@ int grws_csr_to_bcsr_fill(int64_t num_rows, int64_t nnz, const int64_t *window_o
  * builders that must not read a size back): only the first row_ptr[num_rows] entries of col_idx
  * and values exist, nnz_bound >= that count sizes the scratch (grws_csr_to_bcsr_scratch_bytes(
  * num_rows, nnz_bound)) and is what grws_csr_to_bcsr_fill must be given as nnz.
- * num_cols_bound: 0, or a number every column id is below; the builder then sorts keys with a
- * narrower column field (fewer radix passes: it matters for the small blocks of a sampled step). */
+ * num_cols_bound: 0, or a number every column id is below (a hint; the builder does not need it). */
 int grws_csr_to_bcsr_count_bounded(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
                                    const float *values, int64_t nnz_bound, int64_t num_cols_bound,
                                    int64_t *window_offset, void *scratch, size_t scratch_bytes,
