@@ -155,7 +155,7 @@ def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_S
     hop's arrays have the bound sizes of ``sample_layers_sizes`` (the frontier of hop h+1 is the
     whole source list of hop h, its unused tail filled with -1 nodes that sample nothing), so the
     shapes of a step depend only on (number of seeds, fanouts) and recur from step to step.  The
-    call queues about twenty kernels per hop on the current stream and returns; ctypes releases the
+    call queues about ten kernels per hop on the current stream and returns; ctypes releases the
     interpreter lock for its duration, so a sampling thread does not hold up the training thread.
 
     Returns one [window_offset, cols, vals, dst_nodes, src_nodes] list per hop (fanouts in the order
@@ -175,7 +175,8 @@ def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_S
     vals_all = torch.empty(sum(t * 128 for t in tiles) + 8, dtype=values_dtype, device=dev)
     wo_sizes = [(n + 15) // 16 + 1 for n in n_dst]
     wo_all = torch.empty(sum(-(-n // 32) * 32 for n in wo_sizes) + 4 * L, dtype=torch.int64, device=dev)
-    scratch = _scratch(lib.grws_sample_layers_scratch_bytes(seeds.numel(), fan, L, int(pad_to)), dev)
+    num_nodes = row_ptr.numel() - 1
+    scratch = _scratch(lib.grws_sample_layers_sized_scratch_bytes(num_nodes, seeds.numel(), fan, L, int(pad_to)), dev)
     srcs, cols, vals, wos = [], [], [], []
     o32 = ov = ow = 0
     for h in range(L):
@@ -185,8 +186,8 @@ def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_S
         wos.append(wo_all[ow:ow + wo_sizes[h]]); ow += -(-wo_sizes[h] // 32) * 32
     counts = wo_all[ow:ow + 4 * L].view(L, 4) if want_counts else None
     ptrs = lambda ts: (ctypes.c_void_p * L)(*[t.data_ptr() for t in ts])      # noqa: E731
-    _native.check(lib.grws_sample_layers(
-        _ptr(row_ptr), _ptr(col_idx), _ptr(values), _ptr(seeds), seeds.numel(), fan, L,
+    _native.check(lib.grws_sample_layers_sized(
+        _ptr(row_ptr), num_nodes, _ptr(col_idx), _ptr(values), _ptr(seeds), seeds.numel(), fan, L,
         int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(seed_dev), int(pad_to), _DT[values_dtype],
         ptrs(srcs), ptrs(wos), ptrs(cols), ptrs(vals), _ptr(counts) if want_counts else 0,
         scratch.data_ptr(), scratch.numel(), _stream(dev)))

@@ -270,6 +270,150 @@ __global__ void localize_flat_kernel(const int32_t *__restrict__ nbr, int64_t n_
     out_local[e] = u >= 0 ? table_lookup(keys, vals, mask, u) : -1;
 }
 
+// ---------------------------------------------------------------------------------------------
+// dedup of a whole mini-batch over a graph whose node count is known: one hash table for all hops
+// (a hop's destination nodes are the previous hop's source list, so they are in it already), and a
+// bitmap of the node ids per hop instead of a sort of the new ids: a prefix sum of its bit counts
+// gives every new node its place in ascending order.  Ids at or above the node count (a last hop may
+// name some) go to a list of their own and rank behind the others.
+// ---------------------------------------------------------------------------------------------
+constexpr int RANK_THREADS = 256;                // bitmap words per CTA
+
+struct HopRank {
+    uint32_t *bits;                              // [words] new nodes of this hop
+    int32_t *prefix;                             // [words] new nodes in the words before, of the same CTA and all earlier ones
+    int32_t *sums;                               // [CTAs] new nodes of a CTA's words, then of all earlier CTAs
+    int32_t *over;                               // ids past the bitmap
+    int32_t *counters;                           // {new nodes, ids in `over`, CTAs that have counted}
+    int64_t words, num_nodes;
+};
+
+__global__ void layers_init_kernel(int32_t *keys, int32_t *vals, int64_t slots, uint32_t *bits, int64_t n_bits, int32_t *counters, int n_counters) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint4 none = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), fresh = make_uint4(NEW_NODE, NEW_NODE, NEW_NODE, NEW_NODE);
+    for (int64_t i = i0; i < slots / 4; i += stride) {          // slots is a power of two, 64 or more
+        reinterpret_cast<uint4 *>(keys)[i] = none;              // EMPTY_KEY
+        reinterpret_cast<uint4 *>(vals)[i] = fresh;
+    }
+    for (int64_t i = i0; i < n_bits; i += stride) bits[i] = 0;
+    if (i0 < n_counters) counters[i0] = 0;
+}
+
+__global__ void insert_seeds_kernel(const int32_t *__restrict__ seeds, int64_t n, int32_t *keys, int32_t *vals, uint32_t mask) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || seeds[i] < 0) return;
+    bool fresh;
+    const uint32_t h = table_insert(keys, mask, seeds[i], fresh);
+    atomicMin(vals + h, (int32_t)i);             // a repeated seed keeps its first position
+}
+
+__global__ void insert_marked_kernel(const int32_t *__restrict__ nbr, int64_t n_entries, int32_t *keys, uint32_t mask, const HopRank r) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t u = e < n_entries ? nbr[e] : -1;
+    if (u < 0) return;
+    bool fresh;
+    table_insert(keys, mask, u, fresh);
+    if (!fresh) return;
+    if (u < r.num_nodes) atomicOr(r.bits + (u >> 5), 1u << (u & 31));
+    else r.over[atomicAdd(r.counters + 1, 1)] = u;
+}
+
+__device__ __forceinline__ int block_exclusive(int v, int *warp_part, int *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    __syncthreads();                             // the previous use of warp_part is over
+    if (lane == 31) warp_part[warp] = incl;
+    __syncthreads();
+    int ahead = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < RANK_THREADS / 32; ++i) {
+        all += warp_part[i];
+        if (i < warp) ahead += warp_part[i];
+    }
+    *total = all;
+    return ahead + incl - v;
+}
+
+// counts the new nodes of every CTA's words; the CTA that counts last turns the counts into prefixes
+__global__ void __launch_bounds__(RANK_THREADS)
+rank_sums_kernel(const HopRank r) {
+    __shared__ int warp_part[RANK_THREADS / 32];
+    __shared__ bool last;
+    const int64_t i = (int64_t)blockIdx.x * RANK_THREADS + threadIdx.x;
+    int total;
+    const int mine = i < r.words ? __popc(r.bits[i]) : 0;
+    const int before = block_exclusive(mine, warp_part, &total);
+    if (i < r.words) r.prefix[i] = before;
+    if (threadIdx.x == 0) {
+        r.sums[blockIdx.x] = total;
+        __threadfence();
+        last = atomicAdd(r.counters + 2, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int done = 0;
+    for (int b0 = 0; b0 < (int)gridDim.x; b0 += RANK_THREADS) {
+        const int b = b0 + (int)threadIdx.x;
+        const int v = b < (int)gridDim.x ? *reinterpret_cast<const volatile int32_t *>(r.sums + b) : 0;
+        const int ahead = block_exclusive(v, warp_part, &total);
+        if (b < (int)gridDim.x) r.sums[b] = done + ahead;
+        done += total;
+    }
+    if (threadIdx.x == 0) r.counters[0] = done + r.counters[1];
+}
+
+// place of a new node among the hop's new nodes in ascending order
+__device__ __forceinline__ int32_t rank_of(const HopRank &r, int32_t u) {
+    if (u < r.num_nodes) {
+        const int64_t i = u >> 5;
+        return r.sums[i / RANK_THREADS] + r.prefix[i] + __popc(r.bits[i] & ((1u << (u & 31)) - 1u));
+    }
+    const int n_over = r.counters[1];
+    int32_t k = r.counters[0] - n_over;
+    for (int j = 0; j < n_over; ++j) k += r.over[j] < u;
+    return k;
+}
+
+// source list of the hop: destination nodes ++ new nodes in ascending order ++ -1
+__global__ void __launch_bounds__(RANK_THREADS)
+emit_sources_kernel(const HopRank r, const int32_t *__restrict__ dst, int64_t n_dst, int64_t n_src, int32_t *__restrict__ out_src) {
+    const int64_t i = (int64_t)blockIdx.x * RANK_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * RANK_THREADS;
+    if (i < r.words) {
+        uint32_t b = r.bits[i];
+        int32_t *o = out_src + n_dst + r.sums[i / RANK_THREADS] + r.prefix[i];
+        for (; b; b &= b - 1) *o++ = (int32_t)(i * 32) + __ffs(b) - 1;
+    }
+    for (int64_t j = i; j < r.counters[1]; j += stride) out_src[n_dst + rank_of(r, r.over[j])] = r.over[j];
+    for (int64_t j = i; j < n_dst; j += stride) out_src[j] = dst[j];
+    for (int64_t j = n_dst + r.counters[0] + i; j < n_src; j += stride) out_src[j] = -1;
+}
+
+// local id of every sampled neighbour; the table learns the ids of the nodes that are new in this hop
+// (every thread that meets a new node writes the same value)
+__global__ void localize_ranked_kernel(const int32_t *__restrict__ nbr, int64_t n_entries, int64_t n_dst, const int32_t *keys, int32_t *vals,
+                                       uint32_t mask, const HopRank r, int32_t *__restrict__ out_local) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_entries) return;
+    const int32_t u = nbr[e];
+    int32_t l = -1;
+    if (u >= 0) {
+        uint32_t h = hash_node(u) & mask;
+        while (keys[h] != u) h = (h + 1) & mask;             // every neighbour has been inserted
+        l = *reinterpret_cast<const volatile int32_t *>(vals + h);
+        if (l == NEW_NODE) {
+            l = (int32_t)n_dst + rank_of(r, u);
+            *reinterpret_cast<volatile int32_t *>(vals + h) = l;
+        }
+    }
+    out_local[e] = l;
+}
+
 // per-hop figures for the caller: {source nodes (padded destinations + new nodes), sampled edges,
 // tiles of the block, real (non-padding) frontier nodes}
 __global__ void hop_counts_kernel(const int32_t *__restrict__ n_new, const int32_t *__restrict__ dst, int64_t n_dst,
@@ -454,17 +598,25 @@ struct LayersScratch {
     float *w;
     void *dedup, *build;
     size_t dedup_bytes, build_bytes, total;
+    // with a known node count (instead of `dedup`)
+    int32_t *keys, *vals, *counters;
+    uint32_t *bits;                                  // [num_hops * words]
+    HopRank rank;
+    int64_t slots;
 };
 
-static int carve_layers(void *base, int64_t num_seeds, const int *fanouts, int num_hops, int64_t pad_to, LayersScratch *out) {
+static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const int *fanouts, int num_hops, int64_t pad_to, LayersScratch *out) {
     int64_t n_dst[16], n_src[16];
     if (int st = grws_sample_layers_sizes(num_seeds, fanouts, num_hops, pad_to, n_dst, n_src, nullptr)) return st;
     size_t entries = 1, rows = 1, dedup = 0, build = 0;
+    int64_t nodes = 1;
     for (int h = 0; h < num_hops; ++h) {
         const size_t e = (size_t)n_dst[h] * fanouts[h];
         if (e > entries) entries = e;
         if ((size_t)n_dst[h] > rows) rows = (size_t)n_dst[h];
-        const size_t d = carve_dedup(nullptr, n_dst[h], fanouts[h]).total, b = grws_csr_to_bcsr_scratch_bytes(n_dst[h], (int64_t)e);
+        if (n_src[h] > nodes) nodes = n_src[h];
+        const size_t d = num_nodes > 0 ? 0 : carve_dedup(nullptr, n_dst[h], fanouts[h]).total;
+        const size_t b = grws_csr_to_bcsr_scratch_bytes(n_dst[h], (int64_t)e);
         if (d > dedup) dedup = d;
         if (b > build) build = b;
     }
@@ -479,14 +631,34 @@ static int carve_layers(void *base, int64_t num_seeds, const int *fanouts, int n
     out->build = take(build);
     out->dedup_bytes = dedup;
     out->build_bytes = build;
+    if (num_nodes > 0) {
+        int64_t slots = 64;
+        while (slots < 2 * nodes + 16) slots <<= 1;  // every node of the batch: the last source list holds them all
+        const int64_t words = ceil_div(num_nodes, 32);
+        out->slots = slots;
+        out->rank.words = words;
+        out->rank.num_nodes = num_nodes;
+        out->keys = (int32_t *)take((size_t)slots * 4);
+        out->vals = (int32_t *)take((size_t)slots * 4);
+        out->bits = (uint32_t *)take((size_t)words * num_hops * 4);
+        out->counters = (int32_t *)take((size_t)num_hops * 16);
+        out->rank.prefix = (int32_t *)take((size_t)words * 4);
+        out->rank.sums = (int32_t *)take((size_t)ceil_div(words, RANK_THREADS) * 4);
+        out->rank.over = (int32_t *)take(entries * 4);
+    }
     out->total = off;
     return GRWS_OK;
 }
 
 __attribute__((visibility("default")))
 size_t grws_sample_layers_scratch_bytes(int64_t num_seeds, const int *fanouts, int num_hops, int64_t pad_to) {
-    LayersScratch s;
-    if (carve_layers(nullptr, num_seeds, fanouts, num_hops, pad_to, &s) != GRWS_OK) return 0;
+    return grws_sample_layers_sized_scratch_bytes(0, num_seeds, fanouts, num_hops, pad_to);
+}
+
+__attribute__((visibility("default")))
+size_t grws_sample_layers_sized_scratch_bytes(int64_t num_nodes, int64_t num_seeds, const int *fanouts, int num_hops, int64_t pad_to) {
+    LayersScratch s = {};
+    if (num_nodes < 0 || carve_layers(nullptr, num_nodes, num_seeds, fanouts, num_hops, pad_to, &s) != GRWS_OK) return 0;
     return s.total;
 }
 
@@ -496,16 +668,34 @@ int grws_sample_layers(const int64_t *row_ptr, const int32_t *col_idx, const flo
                        int64_t pad_to, int val_dtype, int32_t *const *out_src, int64_t *const *out_window_offset,
                        int32_t *const *out_cols, void *const *out_vals, int64_t *out_counts, void *scratch,
                        size_t scratch_bytes, void *stream) {
+    return grws_sample_layers_sized(row_ptr, 0, col_idx, values, seeds, num_seeds, fanouts, num_hops, seed, seed_dev, pad_to, val_dtype,
+                                    out_src, out_window_offset, out_cols, out_vals, out_counts, scratch, scratch_bytes, stream);
+}
+
+__attribute__((visibility("default")))
+int grws_sample_layers_sized(const int64_t *row_ptr, int64_t num_nodes, const int32_t *col_idx, const float *values,
+                             const int32_t *seeds, int64_t num_seeds, const int *fanouts, int num_hops, uint64_t seed,
+                             const uint64_t *seed_dev, int64_t pad_to, int val_dtype, int32_t *const *out_src,
+                             int64_t *const *out_window_offset, int32_t *const *out_cols, void *const *out_vals, int64_t *out_counts,
+                             void *scratch, size_t scratch_bytes, void *stream) {
+    GRWS_REQUIRE(num_nodes >= 0 && num_nodes < 0x7fffffffLL, "node count outside [0, 2^31)");
     GRWS_REQUIRE(row_ptr && col_idx && (seeds || num_seeds == 0) && out_src && out_window_offset && out_cols && out_vals && scratch,
                  "null pointer");
     GRWS_REQUIRE(val_dtype >= GRWS_F32 && val_dtype <= GRWS_BF16, "bad value dtype %d", val_dtype);
     int64_t n_dst[16], n_src[16], tiles[16];
     if (int st = grws_sample_layers_sizes(num_seeds, fanouts, num_hops, pad_to, n_dst, n_src, tiles)) return st;
-    LayersScratch s;
-    if (int st = carve_layers(scratch, num_seeds, fanouts, num_hops, pad_to, &s)) return st;
+    LayersScratch s = {};
+    if (int st = carve_layers(scratch, num_nodes, num_seeds, fanouts, num_hops, pad_to, &s)) return st;
     if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "sample_layers scratch too small: %zu < %zu", scratch_bytes, s.total);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int32_t *dst = seeds;
+    const uint32_t table_mask = (uint32_t)(s.slots - 1);
+    const unsigned rank_blocks = (unsigned)ceil_div(s.rank.words, RANK_THREADS);
+    if (num_nodes > 0 && num_seeds > 0) {
+        const unsigned nb = nblocks(s.slots / 4, 256);
+        layers_init_kernel<<<nb > 1184 ? 1184 : nb, 256, 0, st>>>(s.keys, s.vals, s.slots, s.bits, s.rank.words * num_hops, s.counters, 4 * num_hops);
+        insert_seeds_kernel<<<nblocks(num_seeds, 256), 256, 0, st>>>(seeds, num_seeds, s.keys, s.vals, table_mask);
+    }
     for (int h = 0; h < num_hops; ++h) {
         const int64_t nd = n_dst[h], f = fanouts[h], n_entries = nd * f, W = ceil_div(nd, (int64_t)TILE_ROWS);
         GRWS_REQUIRE(out_src[h] && out_window_offset[h] && (tiles[h] == 0 || (out_cols[h] && out_vals[h])), "null output of hop %d", h);
@@ -520,23 +710,37 @@ int grws_sample_layers(const int64_t *row_ptr, const int32_t *col_idx, const flo
         sample_hop_kernel<<<nblocks(nd, SAMPLE_WARPS), SAMPLE_WARPS * 32, 0, st>>>(
             row_ptr, col_idx, values, dst, nd, (int)f, seed, seed_dev, (uint32_t)h, s.nbr, s.w, s.cnt);
         // 2. source list = frontier ++ ascending new nodes ++ -1 padding; local id of every neighbour
-        DedupScratch d = carve_dedup(s.dedup, nd, (int)f);
-        const uint32_t mask = d.slots - 1;
-        const int64_t init_n = (int64_t)d.slots > n_src[h] ? (int64_t)d.slots : n_src[h];
-        dedup_init_kernel<<<nblocks(init_n, 256) > 1184 ? 1184 : nblocks(init_n, 256), 256, 0, st>>>(
-            d.keys, d.vals, d.slots, d.cand, n_entries + 1, d.n_new, out_src[h] + nd, n_src[h] - nd);
-        insert_dst_kernel<<<nblocks(nd, 256), 256, 0, st>>>(dst, nd, d.keys, d.vals, mask, out_src[h]);
-        insert_nbr_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, d.keys, d.vals, mask, d.cand, d.n_new);
-        size_t tmp = d.cub_bytes;
-        GRWS_CUDA_TRY(cub::DeviceRadixSort::SortKeys(d.cub_tmp, tmp, d.cand, d.cand_sorted, (int)n_entries, 0, 32, st));
-        rank_new_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(d.cand_sorted, d.n_new, nd, d.keys, d.vals, mask, out_src[h]);
-        localize_flat_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, d.keys, d.vals, mask, s.local);
+        const int32_t *n_new;
+        if (num_nodes > 0) {
+            HopRank r = s.rank;
+            r.bits = s.bits + s.rank.words * h;
+            r.counters = s.counters + 4 * h;
+            insert_marked_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, s.keys, table_mask, r);
+            rank_sums_kernel<<<rank_blocks, RANK_THREADS, 0, st>>>(r);
+            const unsigned emit_blocks = nblocks(n_src[h], 4 * RANK_THREADS);
+            emit_sources_kernel<<<emit_blocks > rank_blocks ? emit_blocks : rank_blocks, RANK_THREADS, 0, st>>>(r, dst, nd, n_src[h], out_src[h]);
+            localize_ranked_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, nd, s.keys, s.vals, table_mask, r, s.local);
+            n_new = r.counters;
+        } else {
+            const DedupScratch d = carve_dedup(s.dedup, nd, (int)f);
+            const uint32_t mask = d.slots - 1;
+            const int64_t init_n = (int64_t)d.slots > n_src[h] ? (int64_t)d.slots : n_src[h];
+            dedup_init_kernel<<<nblocks(init_n, 256) > 1184 ? 1184 : nblocks(init_n, 256), 256, 0, st>>>(
+                d.keys, d.vals, d.slots, d.cand, n_entries + 1, d.n_new, out_src[h] + nd, n_src[h] - nd);
+            insert_dst_kernel<<<nblocks(nd, 256), 256, 0, st>>>(dst, nd, d.keys, d.vals, mask, out_src[h]);
+            insert_nbr_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, d.keys, d.vals, mask, d.cand, d.n_new);
+            size_t tmp = d.cub_bytes;
+            GRWS_CUDA_TRY(cub::DeviceRadixSort::SortKeys(d.cub_tmp, tmp, d.cand, d.cand_sorted, (int)n_entries, 0, 32, st));
+            rank_new_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(d.cand_sorted, d.n_new, nd, d.keys, d.vals, mask, out_src[h]);
+            localize_flat_kernel<<<nblocks(n_entries, 256), 256, 0, st>>>(s.nbr, n_entries, d.keys, d.vals, mask, s.local);
+            n_new = d.n_new;
+        }
         // 3. the hop's BCSR block straight from the fixed-stride lists
         if (int e = grws_block_build_count(s.local, s.w, nd, (int)f, n_src[h], out_window_offset[h], s.build, s.build_bytes, stream)) return e;
         if (int e = block_build_fill(nd, (int)f, out_window_offset[h], tiles[h], out_cols[h], out_vals[h], val_dtype, s.build,
                                      s.build_bytes, st)) return e;
         if (out_counts)
-            hop_counts_kernel<<<1, 1024, 0, st>>>(d.n_new, dst, nd, s.cnt, out_window_offset[h], W, out_counts + 4 * h);
+            hop_counts_kernel<<<1, 1024, 0, st>>>(n_new, dst, nd, s.cnt, out_window_offset[h], W, out_counts + 4 * h);
         GRWS_CUDA_TRY(cudaGetLastError());
         dst = out_src[h];
     }

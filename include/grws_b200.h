@@ -364,6 +364,21 @@ int grws_sample_layers(const int64_t *row_ptr, const int32_t *col_idx, const flo
                        int32_t *const *out_cols, void *const *out_vals, int64_t *out_counts,
                        void *scratch, size_t scratch_bytes, void *stream);
 
+/* The same for a graph of num_nodes nodes (row_ptr has num_nodes + 1 entries): the new nodes of a
+ * hop are put in order through a bitmap of the node ids instead of a sort, with one hash table for
+ * all hops.  num_nodes = 0: not known, as above.  Ids of num_nodes or more stay allowed where the
+ * call above allows them, as neighbours in the last hop. */
+size_t grws_sample_layers_sized_scratch_bytes(int64_t num_nodes, int64_t num_seeds, const int *fanouts,
+                                              int num_hops, int64_t pad_to);
+
+int grws_sample_layers_sized(const int64_t *row_ptr, int64_t num_nodes, const int32_t *col_idx,
+                             const float *values, const int32_t *seeds, int64_t num_seeds,
+                             const int *fanouts, int num_hops, uint64_t seed, const uint64_t *seed_dev,
+                             int64_t pad_to, int val_dtype, int32_t *const *out_src,
+                             int64_t *const *out_window_offset, int32_t *const *out_cols,
+                             void *const *out_vals, int64_t *out_counts, void *scratch,
+                             size_t scratch_bytes, void *stream);
+
 /* ------------------------------------------------------------------------------------------
  * Rows of a feature matrix that is sharded over the GPUs of one node, read from their owners over
  * NVLink with plain loads.  Replaces the reference's placement of large feature matrices in pinned
