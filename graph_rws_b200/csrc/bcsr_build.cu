@@ -30,6 +30,7 @@ constexpr int LARGE_SMEM = BITMAP_WORDS * 4 + BITMAP_WORDS / 2 * 4;   // bits + 
 constexpr int FILL_WARPS = 8;
 constexpr int FILL_BYTES = 4096;                   // tiles a warp assembles in shared memory at a time
 constexpr int FILL_LARGE_THREADS = 512;            // one warp per row of a window
+constexpr int FILL_AHEAD = 8;                      // times 32 entries of a row in flight: a hub's row has thousands (one at a time: 234 us a graph)
 
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
@@ -173,7 +174,7 @@ __device__ __forceinline__ int sort_window(const EntrySource &src, int64_t s, in
 // One warp per window.  Bound by instruction issue (the compare-exchange network: 36 steps of 8 keys a lane
 // for the usual window of up to 256 entries).  Against one radix sort of 64-bit (window, column, row) keys over all
 // entries -- five to seven passes over keys and values, flags, two scans -- a mini-batch of 1,024 seeds and
-// fan-out 15-10-5 is sampled and built in 519 us instead of 769.
+// fan-out 15-10-5 was sampled and built in 519 us instead of 769.
 __global__ void __launch_bounds__(COUNT_WARPS * 32)
 count_windows_kernel(const EntrySource src, int64_t W, BuildScratch s) {
     const int lane = threadIdx.x & 31;
@@ -399,16 +400,25 @@ fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restr
         const int64_t row = w * TILE_ROWS + warp;
         if (row < num_rows) {
             const int64_t end = s.row_start[row + 1];
-            for (int64_t b = s.row_start[row]; b < end; b += 32) {
-                const uint64_t r = b + lane < end ? __ldg(s.rec + b + lane) : ~0ull;
-                const float v = b + lane < end ? __ldg(s.val + b + lane) : 0.f;
-                const uint32_t slot = (uint32_t)r;
-                const unsigned same = __match_any_sync(0xffffffffu, r);
-                if (r != ~0ull && lane == 31 - __clz(same)) {
-                    ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v);
-                    oc[slot] = (int32_t)(r >> 32);
+            for (int64_t b = s.row_start[row]; b < end; b += 32 * FILL_AHEAD) {
+                uint64_t r[FILL_AHEAD];
+                float v[FILL_AHEAD];
+#pragma unroll
+                for (int j = 0; j < FILL_AHEAD; ++j) {
+                    const int64_t i = b + j * 32 + lane;
+                    r[j] = i < end ? __ldg(s.rec + i) : ~0ull;
+                    v[j] = i < end ? __ldg(s.val + i) : 0.f;
                 }
-                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < FILL_AHEAD; ++j) {
+                    const uint32_t slot = (uint32_t)r[j];
+                    const unsigned same = __match_any_sync(0xffffffffu, r[j]);
+                    if (r[j] != ~0ull && lane == 31 - __clz(same)) {
+                        ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v[j]);
+                        oc[slot] = (int32_t)(r[j] >> 32);
+                    }
+                    __syncwarp();
+                }
             }
         }
     }
@@ -425,31 +435,75 @@ template <> __device__ __forceinline__ float to_float<float>(float v) { return v
 template <> __device__ __forceinline__ float to_float<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// one thread per tile element; MODE 0 counts entries per column, MODE 1 scatters them
+// four consecutive values of a tile as floats: one load per lane covers a tile
+__device__ __forceinline__ float4 load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 load4(const __half *p) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 load4(const __nv_bfloat16 *p) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+constexpr int TRANSPOSE_WARPS = 8;
+constexpr int TRANSPOSE_AHEAD = 4;     // tiles a warp has in flight
+
+// MODE 0 counts the non-zero entries per column, MODE 1 scatters them.  The tiles are shared out evenly over the
+// warps, whatever window they belong to: a hub's window has a hundred times the tiles of the others, and
+// with a CTA per window its chain of load, atomic and store was the kernel's time (169 k nodes, 315 k tiles of
+// fp32: counting 283 -> 51 us, scattering 383 -> 134 us; the tiles' bytes alone take 26 us).  vec: cols and vals start on
+// 16-byte boundaries.
 template <typename T, int MODE>
-__global__ void transpose_entries_kernel(int64_t W, const int64_t *__restrict__ window_offset,
-                                         const int32_t *__restrict__ cols, const T *__restrict__ vals,
-                                         int64_t num_cols, int64_t *__restrict__ counts_or_cursor,
-                                         int32_t *__restrict__ out_col, float *__restrict__ out_val) {
-    // one warp per (window, tile): lane handles 4 elements
-    const int64_t w = blockIdx.x;
-    const int64_t t0 = window_offset[w], t1 = window_offset[w + 1];
-    for (int64_t tile = t0 + (threadIdx.x >> 5); tile < t1; tile += blockDim.x >> 5) {
-        const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(TRANSPOSE_WARPS * 32)
+transpose_entries_kernel(int64_t W, const int64_t *__restrict__ window_offset, const int32_t *__restrict__ cols,
+                         const T *__restrict__ vals, int64_t num_cols, int64_t *__restrict__ counts_or_cursor,
+                         int32_t *__restrict__ out_col, float *__restrict__ out_val, bool vec) {
+    const int lane = threadIdx.x & 31;
+    const int64_t n_warps = (int64_t)gridDim.x * TRANSPOSE_WARPS, me = (int64_t)blockIdx.x * TRANSPOSE_WARPS + (threadIdx.x >> 5);
+    const int64_t T0 = __ldg(window_offset + W);
+    int64_t share = (T0 + n_warps - 1) / n_warps;
+    share = (share + TRANSPOSE_AHEAD - 1) / TRANSPOSE_AHEAD * TRANSPOSE_AHEAD;
+    const int64_t t0 = me * share, t1 = t0 + share < T0 ? t0 + share : T0;
+    if (t0 >= t1) return;
+    int64_t w = warp_count_ends_le(window_offset, W, t0, lane);      // the window that holds tile t0
+    int64_t end = __ldg(window_offset + w + 1);
+    for (int64_t t = t0; t < t1; t += TRANSPOSE_AHEAD) {
+        float4 v[TRANSPOSE_AHEAD];
+        int4 c[TRANSPOSE_AHEAD];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int el = lane + 32 * q;                // element of the 16x8 tile
-            const int r = el >> 3, c = el & 7;
-            const int32_t col = cols[tile * TILE_COLS + c];
-            if (col < 0 || col >= num_cols) continue;
-            const float v = to_float<T>(vals[tile * TILE_ELEMS + el]);
-            if (v == 0.0f) continue;
-            if (MODE == 0) {
-                atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + col + 1), 1ull);
-            } else {
-                const int64_t pos = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + col), 1ull);
-                out_col[pos] = (int32_t)(w * TILE_ROWS + r);
-                out_val[pos] = v;
+        for (int q = 0; q < TRANSPOSE_AHEAD; ++q) {
+            v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            c[q] = make_int4(-1, -1, -1, -1);
+            if (t + q < t1) {
+                const T *pv = vals + (t + q) * TILE_ELEMS + lane * 4;
+                const int32_t *pc = cols + (t + q) * TILE_COLS + (lane & 1) * 4;
+                if (vec) {
+                    v[q] = load4(pv);
+                    c[q] = __ldg(reinterpret_cast<const int4 *>(pc));
+                } else {
+                    v[q] = make_float4(to_float<T>(pv[0]), to_float<T>(pv[1]), to_float<T>(pv[2]), to_float<T>(pv[3]));
+                    c[q] = make_int4(pc[0], pc[1], pc[2], pc[3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < TRANSPOSE_AHEAD; ++q) {
+            while (t + q < t1 && t + q >= end) end = __ldg(window_offset + ++w + 1);    // windows without tiles are passed over
+            const float vq[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+            const int32_t cq[4] = {c[q].x, c[q].y, c[q].z, c[q].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (vq[j] == 0.0f || cq[j] < 0 || cq[j] >= num_cols) continue;
+                if (MODE == 0) {
+                    atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j] + 1), 1ull);
+                } else {
+                    const int64_t pos = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j]), 1ull);
+                    out_col[pos] = (int32_t)(w * TILE_ROWS + (lane >> 1));
+                    out_val[pos] = vq[j];
+                }
             }
         }
     }
@@ -532,6 +586,12 @@ static int fill_entries(const BuildScratch &s, int64_t num_rows, int64_t num_til
     return GRWS_OK;
 }
 
+// eight CTAs per SM, fewer where there are not even that many windows' tiles to share out
+static unsigned transpose_blocks(int64_t W) {
+    const int64_t most = 8 * sm_count(), few = ceil_div(W, 2);
+    return (unsigned)(few < most ? (few > 0 ? few : 1) : most);
+}
+
 template <typename T>
 static int transpose_count(const int64_t *wo, const int32_t *cols, const void *vals, int64_t W, int64_t num_cols,
                            int64_t *row_ptr_t, void *scratch, cudaStream_t st) {
@@ -541,7 +601,8 @@ static int transpose_count(const int64_t *wo, const int32_t *cols, const void *v
     cub::DeviceScan::InclusiveSum(nullptr, tmp, (const int64_t *)nullptr, (int64_t *)nullptr, (int)(num_cols + 1));
     GRWS_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)(num_cols + 1) * 8, st));
     if (W > 0)
-        transpose_entries_kernel<T, 0><<<(unsigned)W, 128, 0, st>>>(W, wo, cols, (const T *)vals, num_cols, counts, nullptr, nullptr);
+        transpose_entries_kernel<T, 0><<<transpose_blocks(W), TRANSPOSE_WARPS * 32, 0, st>>>(W, wo, cols, (const T *)vals, num_cols, counts,
+                                                                                             nullptr, nullptr, aligned16(cols) && aligned16(vals));
     GRWS_CUDA_TRY(cub::DeviceScan::InclusiveSum(cub_tmp, tmp, counts, row_ptr_t, (int)(num_cols + 1), st));
     GRWS_CUDA_TRY(cudaGetLastError());
     return GRWS_OK;
@@ -665,15 +726,21 @@ int grws_bcsr_transpose_fill(const int64_t *window_offset, const int32_t *cols, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int64_t *cursor = static_cast<int64_t *>(scratch);
     GRWS_CUDA_TRY(cudaMemcpyAsync(cursor, row_ptr_t, (size_t)(num_cols + 1) * 8, cudaMemcpyDeviceToDevice, st));
-    const unsigned W = (unsigned)num_windows;
-    if (val_dtype == GRWS_F32)
-        transpose_entries_kernel<float, 1><<<W, 128, 0, st>>>(num_windows, window_offset, cols, (const float *)vals, num_cols, cursor, out_col, out_val);
-    else if (val_dtype == GRWS_F16)
-        transpose_entries_kernel<__half, 1><<<W, 128, 0, st>>>(num_windows, window_offset, cols, (const __half *)vals, num_cols, cursor, out_col, out_val);
-    else if (val_dtype == GRWS_BF16)
-        transpose_entries_kernel<__nv_bfloat16, 1><<<W, 128, 0, st>>>(num_windows, window_offset, cols, (const __nv_bfloat16 *)vals, num_cols, cursor, out_col, out_val);
-    else
-        return fail(GRWS_ERR_UNSUPPORTED, "bad value dtype %d", val_dtype);
+    const unsigned nb = transpose_blocks(num_windows);
+    const bool vec = aligned16(cols) && aligned16(vals);
+    switch (val_dtype) {
+        case GRWS_F32:
+            transpose_entries_kernel<float, 1><<<nb, TRANSPOSE_WARPS * 32, 0, st>>>(num_windows, window_offset, cols, (const float *)vals, num_cols, cursor, out_col, out_val, vec);
+            break;
+        case GRWS_F16:
+            transpose_entries_kernel<__half, 1><<<nb, TRANSPOSE_WARPS * 32, 0, st>>>(num_windows, window_offset, cols, (const __half *)vals, num_cols, cursor, out_col, out_val, vec);
+            break;
+        case GRWS_BF16:
+            transpose_entries_kernel<__nv_bfloat16, 1><<<nb, TRANSPOSE_WARPS * 32, 0, st>>>(num_windows, window_offset, cols, (const __nv_bfloat16 *)vals, num_cols, cursor, out_col, out_val, vec);
+            break;
+        default:
+            return fail(GRWS_ERR_UNSUPPORTED, "bad value dtype %d", val_dtype);
+    }
     GRWS_CUDA_TRY(cudaGetLastError());
     return GRWS_OK;
 }
