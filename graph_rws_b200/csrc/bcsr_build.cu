@@ -91,8 +91,8 @@ static BuildScratch carve(void *base, int64_t nnz, int64_t num_rows) {
 }
 
 // Ascending bitonic sort of 32 * E keys held by one warp; key i is k[i % E] of lane i / E.
-template <int E>
-__device__ __forceinline__ void warp_sort(uint64_t (&k)[E], int lane) {
+template <int E, typename Key>
+__device__ __forceinline__ void warp_sort(Key (&k)[E], int lane) {
 #pragma unroll
     for (int size = 2; size <= 32 * E; size <<= 1) {
 #pragma unroll
@@ -103,79 +103,103 @@ __device__ __forceinline__ void warp_sort(uint64_t (&k)[E], int lane) {
                 const bool keep_min = ((lane & ls) == 0) == up;
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
-                    const uint64_t o = __shfl_xor_sync(0xffffffffu, k[e], ls);
-                    k[e] = (k[e] < o) == keep_min ? k[e] : o;
+                    const Key o = __shfl_xor_sync(0xffffffffu, k[e], ls);
+                    k[e] = keep_min ? min(k[e], o) : max(k[e], o);
                 }
             } else {
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
                     if (e & stride) continue;
                     const bool up = size < E ? (e & size) == 0 : (lane & (size / E)) == 0;
-                    const uint64_t a = k[e], b = k[e + stride];
-                    const bool swap = (a > b) == up;
-                    k[e] = swap ? b : a;
-                    k[e + stride] = swap ? a : b;
+                    const Key lo = min(k[e], k[e + stride]), hi = max(k[e], k[e + stride]);
+                    k[e] = up ? lo : hi;
+                    k[e + stride] = up ? hi : lo;
                 }
             }
         }
     }
 }
 
-// Sorts one window's `m` entries, gives every distinct column its slot and writes the records in
-// order.  `ends`: in lanes 0..15, where the entries of that row end, counted from the window's first.
-template <int E>
-__device__ __forceinline__ int sort_window(const EntrySource &src, int64_t s, int m, int ends, int lane,
+// Gives every distinct column of one window its slot and writes the records in order.  A key is
+// column << POS_BITS | position; the rows ascend with the position, so this is also the order by (column, row,
+// position).  `ends`: in lanes 0..15, where the entries of that row end, counted from the window's first.
+constexpr int POS_BITS = 9;                                           // SMALL_ENTRIES positions
+template <int E, typename Key>
+__device__ __forceinline__ int rank_window(Key (&k)[E], const EntrySource &src, int64_t s, int m, int ends, int lane,
                                            uint64_t *__restrict__ rec, float *__restrict__ val) {
-    constexpr uint64_t NONE = ~0ull;
-    uint64_t k[E];                                                    // column 32 | row 4 | position 12
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int p = e * 32 + lane;
-        const int32_t c = p < m ? __ldg(src.col + s + p) : 0;
+    constexpr Key NONE = ~Key(0);
+    warp_sort<E, Key>(k, lane);
+    const Key before = __shfl_up_sync(0xffffffffu, k[E - 1], 1), after = __shfl_down_sync(0xffffffffu, k[0], 1);
+    auto row_of = [&](Key key) {                                      // number of rows that end at or before the entry
+        const int p = (int)(key & ((1u << POS_BITS) - 1u));
         int row = 0;
 #pragma unroll
-        for (int step = TILE_ROWS / 2; step > 0; step >>= 1)          // number of rows that end at or before p
-            row += p >= __shfl_sync(0xffffffffu, ends, row + step - 1) ? step : 0;
-        k[e] = p < m && !src.empty(c) ? (uint64_t)(uint32_t)c << 16 | (uint64_t)(row << 12 | p) : NONE;
-    }
-    warp_sort<E>(k, lane);
-    const uint64_t before = __shfl_up_sync(0xffffffffu, k[E - 1], 1), after = __shfl_down_sync(0xffffffffu, k[0], 1);
-    int heads = 0;
-    bool head[E];
+        for (int step = TILE_ROWS / 2; step > 0; step >>= 1) row += p >= __shfl_sync(0xffffffffu, ends, row + step - 1) ? step : 0;
+        return row;
+    };
+    uint32_t heads = 0;                                               // bit e: key e opens a column
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const bool first = e == 0 && lane == 0;
-        const uint64_t prev = e == 0 ? before : k[e > 0 ? e - 1 : 0];
-        head[e] = k[e] != NONE && (first || (prev >> 16) != (k[e] >> 16));
-        heads += head[e];
+        const Key prev = e == 0 ? before : k[e > 0 ? e - 1 : 0];
+        if (k[e] != NONE && ((e == 0 && lane == 0) || (prev >> POS_BITS) != (k[e] >> POS_BITS))) heads |= 1u << e;
     }
-    int incl = heads;
+    int incl = __popc(heads);
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const int o = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += o;
     }
-    int slot = incl - heads - 1;
+    int slot = incl - 1, next_row = __shfl_down_sync(0xffffffffu, row_of(k[0]), 1);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int i = lane * E + e;
-        slot += head[e];
-        if (i >= m) continue;
-        const bool last = e == E - 1 && lane == 31;
-        const uint64_t next = last ? NONE : (e == E - 1 ? after : k[e < E - 1 ? e + 1 : 0]);
-        const bool drop = k[e] == NONE || (next != NONE && (next >> 12) == (k[e] >> 12));
-        const uint32_t col = (uint32_t)(k[e] >> 16), row = (uint32_t)(k[e] >> 12) & (TILE_ROWS - 1);
-        rec[s + i] = (uint64_t)col << 32 | (uint64_t)((uint32_t)slot << 5 | row << 1 | (drop ? 1u : 0u));
-        val[s + i] = drop ? 0.f : __ldg(src.val + s + (int)(k[e] & 0xfff));
+    for (int e = E - 1; e >= 0; --e) {
+        const int i = lane * E + e, row = row_of(k[e]);
+        const Key next = e == E - 1 ? (lane == 31 ? NONE : after) : k[e < E - 1 ? e + 1 : 0];
+        const bool drop = k[e] == NONE || (next != NONE && (next >> POS_BITS) == (k[e] >> POS_BITS) && next_row == row);
+        if (i < m) {
+            const uint32_t col = (uint32_t)(k[e] >> POS_BITS);
+            rec[s + i] = (uint64_t)col << 32 | (uint64_t)((uint32_t)slot << 5 | (uint32_t)row << 1 | (drop ? 1u : 0u));
+            val[s + i] = drop ? 0.f : __ldg(src.val + s + (int)(k[e] & ((1u << POS_BITS) - 1u)));
+        }
+        slot -= heads >> e & 1u;
+        next_row = row;
     }
     return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// Keys of 32 bits where the window's columns leave room for the position (ids below 2^23 - 1: a min or max is one
+// instruction then, and a key one shuffle), of 64 bits otherwise.  Both directions of a 169 k-node graph: 153 us with
+// 64-bit keys throughout, 87 us with 32-bit ones.
+template <int E>
+__device__ __forceinline__ int sort_window(const EntrySource &src, int64_t s, int m, int ends, int lane,
+                                           uint64_t *__restrict__ rec, float *__restrict__ val) {
+    uint32_t c[E], live = 0, top = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int p = e * 32 + lane;
+        const int32_t x = p < m ? __ldg(src.col + s + p) : 0;
+        c[e] = (uint32_t)x;
+        if (p < m && !src.empty(x)) {
+            live |= 1u << e;
+            top = max(top, c[e]);
+        }
+    }
+    if (__reduce_max_sync(0xffffffffu, top) < (1u << (32 - POS_BITS)) - 1u) {
+        uint32_t k[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) k[e] = live >> e & 1u ? c[e] << POS_BITS | (uint32_t)(e * 32 + lane) : ~0u;
+        return rank_window<E, uint32_t>(k, src, s, m, ends, lane, rec, val);
+    }
+    unsigned long long k[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) k[e] = live >> e & 1u ? (unsigned long long)c[e] << POS_BITS | (uint32_t)(e * 32 + lane) : ~0ull;
+    return rank_window<E, unsigned long long>(k, src, s, m, ends, lane, rec, val);
 }
 
 // One warp per window.  Bound by instruction issue (the compare-exchange network: 36 steps of 8 keys a lane
 // for the usual window of up to 256 entries).  Against one radix sort of 64-bit (window, column, row) keys over all
 // entries -- five to seven passes over keys and values, flags, two scans -- a mini-batch of 1,024 seeds and
 // fan-out 15-10-5 was sampled and built in 519 us instead of 769.
-__global__ void __launch_bounds__(COUNT_WARPS * 32)
+__global__ void __launch_bounds__(COUNT_WARPS * 32, 3)
 count_windows_kernel(const EntrySource src, int64_t W, BuildScratch s) {
     const int lane = threadIdx.x & 31;
     const int64_t w = (int64_t)blockIdx.x * COUNT_WARPS + (threadIdx.x >> 5);
