@@ -1,0 +1,46 @@
+"""The sampler's lane groups at their edges, and the batch-wide node table: bit-exact against the host replay."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(n, top, num_cols, seed):
+    rng = np.random.default_rng(seed)
+    deg = rng.integers(0, top, n)
+    rp = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    return rp, rng.integers(0, num_cols, rp[-1]).astype(np.int32), rng.standard_normal(rp[-1]).astype(np.float32)
+
+
+@pytest.mark.parametrize("fanout", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33])
+def test_hop_groups(oracle, fanout):
+    from graph_rws_b200 import core
+    rp, ci, vv = _csr(333, 4 * fanout + 2, 333, fanout)
+    nodes = np.concatenate([np.arange(333), [-1, 5, -1]]).astype(np.int32)
+    got = core.sample_hop(*(torch.from_numpy(a).cuda() for a in (rp, ci, vv, nodes)), fanout, seed=11, hop=2)
+    for a, b in zip(got, oracle.sample_hop(rp, ci, vv, nodes, fanout, 11, 2)):
+        assert np.array_equal(a.cpu().numpy().reshape(-1), np.asarray(b).reshape(-1))
+
+
+@pytest.mark.parametrize("n,num_cols,fanouts", [
+    (40, 40, [3, 2, 2]),            # one bitmap word and a bit; sources soon cover the graph
+    (8192, 8192, [4, 3]),           # exactly one CTA's words
+    (20011, 20011, [5, 4]),         # several CTAs, a ragged last word
+    (64, 9000, [7]),                # a last hop that names ids past the node count
+])
+def test_batch_table(oracle, n, num_cols, fanouts):
+    from graph_rws_b200 import core
+    rp, ci, vv = _csr(n, 12, num_cols, n)
+    seeds = np.random.default_rng(1).integers(0, n, 33).astype(np.int32)         # some of them twice
+    hops = core.sample_layers_fused(*(torch.from_numpy(a).cuda() for a in (rp, ci, vv, seeds)), fanouts, seed=9)
+    dst = seeds
+    for h, f in enumerate(fanouts):
+        wo, cols, vals, _, src = (t.cpu().numpy() for t in hops[h])
+        nbr, w, _ = oracle.sample_hop(rp, ci, vv, dst, f, 9, h)
+        src_r, wo_r, cols_r, vals_r = oracle.build_block(dst, nbr, w)
+        assert np.array_equal(src[:src_r.size], src_r) and (src[src_r.size:] == -1).all()
+        assert np.array_equal(wo, wo_r)
+        assert np.array_equal(cols[:cols_r.size], cols_r) and (cols[cols_r.size:] == -1).all()
+        assert np.array_equal(vals[:vals_r.size], vals_r) and (vals[vals_r.size:] == 0).all()
+        dst = src
