@@ -30,7 +30,7 @@ constexpr int LARGE_SMEM = BITMAP_WORDS * 4 + BITMAP_WORDS / 2 * 4;   // bits + 
 constexpr int FILL_WARPS = 8;
 constexpr int FILL_BYTES = 4096;                   // tiles a warp assembles in shared memory at a time
 constexpr int FILL_LARGE_THREADS = 512;            // one warp per row of a window
-constexpr int FILL_AHEAD = 8;                      // times 32 entries of a row in flight: a hub's row has thousands (one at a time: 234 us a graph)
+constexpr int FILL_AHEAD = 16;                     // times 32 entries of a row in flight: a hub's row has thousands (one at a time: 234 us a graph)
 
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
@@ -435,8 +435,11 @@ fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restr
                 }
 #pragma unroll
                 for (int j = 0; j < FILL_AHEAD; ++j) {
-                    const uint32_t slot = (uint32_t)r[j];
-                    const unsigned same = __match_any_sync(0xffffffffu, r[j]);
+                    const uint32_t slot = (uint32_t)r[j];                 // all ones in an empty entry, no slot is
+                    // slots that ascend from lane to lane are distinct: sorted rows need no look for duplicates
+                    const uint32_t before = __shfl_up_sync(0xffffffffu, slot, 1);
+                    unsigned same = 1u << lane;
+                    if (__any_sync(0xffffffffu, lane > 0 && before >= slot)) same = __match_any_sync(0xffffffffu, slot);
                     if (r[j] != ~0ull && lane == 31 - __clz(same)) {
                         ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v[j]);
                         oc[slot] = (int32_t)(r[j] >> 32);
@@ -574,6 +577,37 @@ static int sm_count() {
     return sms;
 }
 
+// Inclusive prefix sum by one CTA.  Up to SCAN_ONE numbers (131,000 rows) one launch of this takes the time of the
+// first of the device-wide scan's two.
+constexpr int SCAN_THREADS = 1024, SCAN_ONE = 8 * SCAN_THREADS;
+__global__ void __launch_bounds__(SCAN_THREADS)
+scan_one_kernel(const int64_t *__restrict__ in, int64_t *__restrict__ out, int n) {
+    __shared__ int64_t part[SCAN_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int each = (n + SCAN_THREADS - 1) / SCAN_THREADS, i0 = threadIdx.x * each;
+    int64_t v[SCAN_ONE / SCAN_THREADS], sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ONE / SCAN_THREADS; ++k) {
+        v[k] = k < each && i0 + k < n ? in[i0 + k] : 0;
+        sum += v[k];
+    }
+    int64_t incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int64_t o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    int64_t at = incl - sum;
+    for (int k = 0; k < warp; ++k) at += part[k];
+#pragma unroll
+    for (int k = 0; k < SCAN_ONE / SCAN_THREADS; ++k) {
+        at += v[k];
+        if (k < each && i0 + k < n) out[i0 + k] = at;
+    }
+}
+
 // Count phase of both front ends.  may_be_large: some window may have more than SMALL_ENTRIES entries.
 static int count_entries(const BuildScratch &s, const EntrySource &src, int64_t W, bool may_be_large, int64_t *window_offset,
                          cudaStream_t st) {
@@ -588,8 +622,12 @@ static int count_entries(const BuildScratch &s, const EntrySource &src, int64_t 
         const int64_t grid = 2 * sm_count();
         count_large_kernel<<<(unsigned)(W < grid ? W : grid), LARGE_THREADS, LARGE_SMEM, st>>>(src, s);
     }
-    size_t tmp = s.cub_bytes;
-    GRWS_CUDA_TRY(cub::DeviceScan::InclusiveSum(s.cub_tmp, tmp, s.tiles, window_offset, (int)(W + 1), st));
+    if (W + 1 <= SCAN_ONE) {
+        scan_one_kernel<<<1, SCAN_THREADS, 0, st>>>(s.tiles, window_offset, (int)(W + 1));
+    } else {
+        size_t tmp = s.cub_bytes;
+        GRWS_CUDA_TRY(cub::DeviceScan::InclusiveSum(s.cub_tmp, tmp, s.tiles, window_offset, (int)(W + 1), st));
+    }
     GRWS_CUDA_TRY(cudaGetLastError());
     return GRWS_OK;
 }
