@@ -278,7 +278,8 @@ def spmm_transpose(window_offset, original_col_indices, values_condensed, grad_o
     return out[:num_cols]
 
 
-from .sampling import (SamplingTimingResult, bcsr_to_csr, build_block, reindex_bcsr,  # noqa: E402,F401
+from .sampling import (SamplingTimingResult, bcsr_to_csr, build_block, reindex_bcsr, relabel_columns,  # noqa: E402,F401
+                       sanitize_columns,
                        sample_all_layers, sample_hop, sample_layers_csr, sample_layers_fused,
                        sample_layers_sizes)
 

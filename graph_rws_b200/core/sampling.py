@@ -256,3 +256,28 @@ def reindex_bcsr(col_indices, values_condensed, active_windows, tile_rows=16, ti
                                         _ptr(active_windows), col_indices.numel(), active_windows.numel(),
                                         int(tile_rows), int(tile_cols), _ptr(out), _stream(col_indices.device)))
     return out
+
+
+def relabel_columns(cols, node_ids):
+    """``node_ids[cols]`` for the non-negative ids of ``cols`` (int32), the others as they are."""
+    if not (cols.is_cuda and cols.dtype == node_ids.dtype == torch.int32 and node_ids.device == cols.device):
+        return torch.where(cols >= 0, node_ids[cols.clamp(min=0).long()], cols)
+    cols, node_ids = cols.contiguous(), node_ids.contiguous()
+    out = torch.empty_like(cols)
+    _native.check(_native.lib().grws_relabel_columns(_ptr(cols), cols.numel(), _ptr(node_ids), node_ids.numel(), _ptr(out),
+                                                     _stream(cols.device)))
+    return out
+
+
+def sanitize_columns(cols, values, num_cols):
+    """In place: ids of -1 or ``num_cols`` and more become 0, their column of the 16x8 tile zero."""
+    if not (cols.is_cuda and values.device == cols.device and cols.dtype == torch.int32 and values.dtype in _DT
+            and cols.is_contiguous() and values.is_contiguous()):
+        bad = (cols == -1) | (cols >= num_cols)
+        cols.masked_fill_(bad, 0)
+        values.view(-1, 16, 8).masked_fill_(bad.view(-1, 1, 8), 0.0)
+        return
+    _native.check(_native.lib().grws_sanitize_columns(_ptr(cols), _ptr(values), _DT[values.dtype], cols.numel() // 8, int(num_cols),
+                                                      _stream(cols.device)))
+    torch.autograd.graph.increment_version(cols)          # what is cached for the old contents goes
+    torch.autograd.graph.increment_version(values)

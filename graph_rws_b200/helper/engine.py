@@ -119,6 +119,8 @@ def layer0_inputs(blocks, features, fetch_rows=None):
     multiplies and gathers over every row of the matrix instead (layers/layer.py:40,
     helper/engine.py:170-171)."""
     import copy
+
+    from .. import core
     b0 = blocks[0]
     if fetch_rows is not None:
         ids = b0.input_nodes
@@ -130,8 +132,7 @@ def layer0_inputs(blocks, features, fetch_rows=None):
         x[real] = rows
         return blocks, x
     g0 = copy.copy(b0)
-    cols = b0.original_col_indices
-    g0.original_col_indices = torch.where(cols >= 0, b0.input_nodes[cols.clamp(min=0).long()], cols)
+    g0.original_col_indices = core.relabel_columns(b0.original_col_indices, b0.input_nodes)
     g0.self_rows = b0.output_nodes.clamp(min=0).long()
     g0.num_cols = features.shape[0]
     g0._shared = {}

@@ -84,11 +84,7 @@ class GCN_BCSR(nn.Module):
         state = (g.original_col_indices.data_ptr(), g.values_condensed.data_ptr())
         if shared is not None and shared.get(key) == state:
             return
-        cols = g.original_col_indices
-        bad = (cols == -1) | (cols >= num_src)
-        cols.masked_fill_(bad, 0)
-        vals = g.values_condensed.view(-1, g.tile_rows, g.tile_cols)
-        vals.masked_fill_(bad.view(-1, 1, g.tile_cols), 0.0)
+        core.sanitize_columns(g.original_col_indices, g.values_condensed, num_src)
         if shared is not None:
             shared[key] = state
 
