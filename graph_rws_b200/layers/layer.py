@@ -121,10 +121,18 @@ class BCSRGraphConv(nn.Module):
         target_rows = h_neigh.shape[0]
         if features_target is not None:
             h_in_self = features_target
-        elif features.shape[0] >= target_rows:
-            h_in_self = features[:target_rows]          # target nodes first
         else:
-            h_in_self = F.pad(features, (0, 0, 0, target_rows - features.shape[0]))
+            h_in_self = features[:target_rows]          # target nodes first
+        if (not torch.is_grad_enabled() and not torch.is_autocast_enabled() and h_in_self.shape[0] <= target_rows
+                and h_neigh.dtype == h_in_self.dtype == w_self.dtype):
+            # nothing is recorded: the GEMM adds to the product's rows itself, which saves the pass that
+            # adds the two and, where the rows of the last window are missing, a padded copy of the input
+            if features_target is not None:
+                h_neigh = h_neigh[:h_in_self.shape[0]]
+            h_neigh[:h_in_self.shape[0]].addmm_(h_in_self, w_self)
+            return h_neigh[:, :self.out_feats] if pad else h_neigh
+        if h_in_self.shape[0] < target_rows and features_target is None:
+            h_in_self = F.pad(h_in_self, (0, 0, 0, target_rows - h_in_self.shape[0]))
         h_self = torch.matmul(h_in_self, w_self)
         # the SpMM returns whole windows (W*16 rows); trim or pad to the self path
         if h_neigh.shape[0] > h_self.shape[0]:
