@@ -516,20 +516,32 @@ transpose_entries_kernel(int64_t W, const int64_t *__restrict__ window_offset, c
                 }
             }
         }
+        // all atomics of the tiles in flight first, then the stores that wait for their results
+        int32_t row[TRANSPOSE_AHEAD];
+        int64_t pos[TRANSPOSE_AHEAD][4];
 #pragma unroll
         for (int q = 0; q < TRANSPOSE_AHEAD; ++q) {
             while (t + q < t1 && t + q >= end) end = __ldg(window_offset + ++w + 1);    // windows without tiles are passed over
+            row[q] = (int32_t)(w * TILE_ROWS + (lane >> 1));
             const float vq[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
             const int32_t cq[4] = {c[q].x, c[q].y, c[q].z, c[q].w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+                pos[q][j] = -1;
                 if (vq[j] == 0.0f || cq[j] < 0 || cq[j] >= num_cols) continue;
-                if (MODE == 0) {
-                    atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j] + 1), 1ull);
-                } else {
-                    const int64_t pos = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j]), 1ull);
-                    out_col[pos] = (int32_t)(w * TILE_ROWS + (lane >> 1));
-                    out_val[pos] = vq[j];
+                if (MODE == 0) atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j] + 1), 1ull);
+                else pos[q][j] = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(counts_or_cursor + cq[j]), 1ull);
+            }
+        }
+        if (MODE == 1) {
+#pragma unroll
+            for (int q = 0; q < TRANSPOSE_AHEAD; ++q) {
+                const float vq[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (pos[q][j] < 0) continue;
+                    out_col[pos[q][j]] = row[q];
+                    out_val[pos[q][j]] = vq[j];
                 }
             }
         }
