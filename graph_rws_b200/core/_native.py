@@ -42,6 +42,7 @@ SIGNATURES = {
     "grws_spmm_set_wait_limit": (c_i32, [ctypes.c_longlong]),
     "grws_csr_to_bcsr_scratch_bytes": (c_sz, [c_i64, c_i64]),
     "grws_csr_to_bcsr_count": (c_i32, [c_i64, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp, c_sz, c_vp]),
+    "grws_csr_to_bcsr_count_unique": (c_i32, [c_i64, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp, c_sz, c_vp]),
     "grws_csr_to_bcsr_fill": (c_i32, [c_i64, c_i64, c_vp, c_i64, c_vp, c_vp, c_i32, c_vp, c_sz, c_vp]),
     "grws_csr_to_bcsr_count_bounded": (c_i32, [c_i64, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_sz, c_vp]),
     "grws_block_build_count": (c_i32, [c_vp, c_vp, c_i64, c_i32, c_i64, c_vp, c_vp, c_sz, c_vp]),

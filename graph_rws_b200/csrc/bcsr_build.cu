@@ -27,10 +27,11 @@ constexpr int COUNT_WARPS = 8;
 constexpr int LARGE_THREADS = 1024;
 constexpr int BITMAP_WORDS = 16384;                // 524,288 columns per round of a large window
 constexpr int LARGE_SMEM = BITMAP_WORDS * 4 + BITMAP_WORDS / 2 * 4;   // bits + one prefix per word pair: two CTAs per SM
+constexpr int LARGE_PLAIN = 1 << 30;               // flag in BuildScratch::large (there are fewer than 2^28 windows)
 constexpr int FILL_WARPS = 8;
 constexpr int FILL_BYTES = 4096;                   // tiles a warp assembles in shared memory at a time
 constexpr int FILL_LARGE_THREADS = 512;            // one warp per row of a window
-constexpr int FILL_AHEAD = 16;                     // times 32 entries of a row in flight: a hub's row has thousands (one at a time: 234 us a graph)
+constexpr int FILL_AHEAD = 8;                      // times 32 entries of a row in flight where their order is kept (a hub's row has thousands)
 
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
@@ -42,6 +43,7 @@ struct EntrySource {
     const float *val;
     int64_t num_rows;
     int fanout;
+    bool unique;            // the caller knows that no (row, column) pair occurs twice
     __device__ __forceinline__ int64_t row_start(int64_t r) const {
         r = r < num_rows ? r : num_rows;
         return row_ptr ? row_ptr[r] : r * fanout;
@@ -60,7 +62,10 @@ struct BuildScratch {
     float *val;             // value of the entry rec describes
     int32_t *row_start;     // [num_rows + 1]
     int64_t *tiles;         // [W+1] tiles per window, shifted by one
-    int32_t *large;         // [1 + W] number of large windows, then their ids in no fixed order
+    int32_t *large;         // [1 + W] number of large windows, then their ids in no fixed order (bit 30: its entries are
+                            // all distinct, so they can be written in any order)
+    int32_t *columns;       // [W] distinct columns of the large window listed at that place
+    int32_t *ucol;          // column of every slot of a large window, from its first entry's place on
     void *cub_tmp;
     size_t cub_bytes;
     size_t total;
@@ -84,6 +89,8 @@ static BuildScratch carve(void *base, int64_t nnz, int64_t num_rows) {
     s.row_start = (int32_t *)take((size_t)(num_rows + 1) * 4);
     s.tiles = (int64_t *)take((size_t)(W + 1) * 8);
     s.large = (int32_t *)take((size_t)(W + 1) * 4);
+    s.columns = (int32_t *)take((size_t)(W + 1) * 4);
+    s.ucol = (int32_t *)take(n * 4);
     s.cub_bytes = scan_temp_bytes(W + 1);
     s.cub_tmp = take(s.cub_bytes);
     s.total = off;
@@ -241,6 +248,7 @@ __global__ void __launch_bounds__(LARGE_THREADS, 2)
 count_large_kernel(const EntrySource src, BuildScratch s) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t warp_part[LARGE_THREADS / 32];
+    __shared__ int out_of_order;
     uint32_t *bits = smem, *prefix = smem + BITMAP_WORDS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_large = s.large[0];
@@ -303,7 +311,9 @@ count_large_kernel(const EntrySource src, BuildScratch s) {
             for (int i = p0; i < p1; ++i) {
                 const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
                 prefix[i] = at;
-                at += __popc(v.x) + __popc(v.y);
+                const uint32_t c0 = lo + (uint32_t)i * 64;
+                for (uint32_t b = v.x; b; b &= b - 1) s.ucol[first + at++] = (int32_t)(c0 + __ffs(b) - 1);
+                for (uint32_t b = v.y; b; b &= b - 1) s.ucol[first + at++] = (int32_t)(c0 + 31 + __ffs(b));
             }
             __syncthreads();
             for (int64_t i = tid; i < m; i += LARGE_THREADS) {
@@ -320,11 +330,28 @@ count_large_kernel(const EntrySource src, BuildScratch s) {
             if (more) lo = block_reduce(next, true, warp_part);
             __syncthreads();                                          // bits and prefix are free again
         }
+        // values; and are the rows in strictly ascending order, that is: does every place where the columns do not
+        // ascend lie between two rows
+        if (tid == 0) out_of_order = 0;
+        __syncthreads();
+        int odd = 0;
         for (int64_t i = tid; i < m; i += LARGE_THREADS) {
-            if (src.empty(__ldg(col + i))) s.rec[first + i] = ~0ull;
+            const int32_t c = __ldg(col + i);
+            if (src.empty(c)) s.rec[first + i] = ~0ull;
+            if (i + 1 < m && (uint32_t)c >= (uint32_t)__ldg(col + i + 1)) ++odd;
             s.val[first + i] = __ldg(src.val + first + i);
         }
-        if (tid == 0) s.tiles[w + 1] = ((int64_t)total + TILE_COLS - 1) / TILE_COLS;
+        if (tid > 0 && tid < TILE_ROWS) {
+            const int64_t at = src.row_start(w * TILE_ROWS + tid) - first, before = src.row_start(w * TILE_ROWS + tid - 1) - first;
+            if (at > before && at < m && (uint32_t)__ldg(col + at - 1) >= (uint32_t)__ldg(col + at)) --odd;
+        }
+        if (odd) atomicAdd(&out_of_order, odd);
+        __syncthreads();
+        if (tid == 0) {
+            s.tiles[w + 1] = ((int64_t)total + TILE_COLS - 1) / TILE_COLS;
+            s.columns[q] = (int32_t)total;
+            s.large[1 + q] = (int32_t)w | (src.row_ptr && (src.unique || out_of_order == 0) ? LARGE_PLAIN : 0);
+        }
     }
 }
 
@@ -404,48 +431,73 @@ fill_windows_kernel(int64_t W, int64_t num_rows, int64_t num_tiles, const BuildS
         store_piece(out_cols, i, make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), vec);
 }
 
-// Large windows, one CTA each: empty tiles, then a warp per row scatters that row's entries in their order,
-// so that the last of several entries of one column is the one that stays.
+// Large windows, one CTA each: column ids and empty tiles, then the entries are scattered.  Distinct entries go in any
+// order, all threads side by side; otherwise a warp per row keeps their order, so that the last of several entries of
+// one column is the one that stays.  Bound by the scattered stores of the CTA with the most entries: a hub's row has
+// thousands and its 15 neighbours few, so a warp per row leaves 15 of 16 warps waiting.  A 169 k-node graph and its
+// transpose, fp32: 648 us built with a warp per row throughout, 548 us with distinct entries side by side.
 template <typename T>
 __global__ void __launch_bounds__(FILL_LARGE_THREADS)
 fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restrict__ window_offset,
                   int32_t *__restrict__ out_cols, T *__restrict__ out_vals, bool vec) {
     constexpr int TILE_V = TILE_ELEMS * (int)sizeof(T) / 16;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int32_t start[TILE_ROWS + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_large = s.large[0];
     for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
-        const int64_t w = s.large[1 + q], t0 = window_offset[w], nt = window_offset[w + 1] - t0;
+        const int32_t id = s.large[1 + q];
+        const bool plain = id & LARGE_PLAIN;
+        const int64_t w = id & ~LARGE_PLAIN, t0 = window_offset[w], nt = window_offset[w + 1] - t0;
+        __syncthreads();                                  // the previous window's use of `start` is over
+        if (tid <= TILE_ROWS) {
+            const int64_t row = w * TILE_ROWS + tid;
+            start[tid] = s.row_start[row < num_rows ? row : num_rows];
+        }
+        __syncthreads();
+        const int first = start[0], end = start[TILE_ROWS], columns = s.columns[q];
         T *ov = out_vals + t0 * TILE_ELEMS;
         int32_t *oc = out_cols + t0 * TILE_COLS;
-        for (int64_t i = threadIdx.x; i < nt * TILE_V; i += FILL_LARGE_THREADS) store_piece(ov, i, make_uint4(0u, 0u, 0u, 0u), vec);
-        for (int64_t i = threadIdx.x; i < nt * 2; i += FILL_LARGE_THREADS)
-            store_piece(oc, i, make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), vec);
+        for (int64_t i = tid; i < nt * TILE_V; i += FILL_LARGE_THREADS) store_piece(ov, i, make_uint4(0u, 0u, 0u, 0u), vec);
+        for (int64_t i = tid; i < nt * TILE_COLS; i += FILL_LARGE_THREADS) oc[i] = i < columns ? __ldg(s.ucol + first + i) : -1;
         __syncthreads();
-        const int64_t row = w * TILE_ROWS + warp;
-        if (row < num_rows) {
-            const int64_t end = s.row_start[row + 1];
-            for (int64_t b = s.row_start[row]; b < end; b += 32 * FILL_AHEAD) {
-                uint64_t r[FILL_AHEAD];
-                float v[FILL_AHEAD];
+        if (plain) {
+            for (int64_t b = first; b < end; b += FILL_LARGE_THREADS * 4) {
+                uint32_t slot[4];
+                float v[4];
 #pragma unroll
-                for (int j = 0; j < FILL_AHEAD; ++j) {
-                    const int64_t i = b + j * 32 + lane;
-                    r[j] = i < end ? __ldg(s.rec + i) : ~0ull;
+                for (int j = 0; j < 4; ++j) {
+                    const int64_t i = b + j * FILL_LARGE_THREADS + tid;
+                    slot[j] = i < end ? (uint32_t)__ldg(s.rec + i) : 0u;
                     v[j] = i < end ? __ldg(s.val + i) : 0.f;
                 }
 #pragma unroll
-                for (int j = 0; j < FILL_AHEAD; ++j) {
-                    const uint32_t slot = (uint32_t)r[j];                 // all ones in an empty entry, no slot is
-                    // slots that ascend from lane to lane are distinct: sorted rows need no look for duplicates
-                    const uint32_t before = __shfl_up_sync(0xffffffffu, slot, 1);
-                    unsigned same = 1u << lane;
-                    if (__any_sync(0xffffffffu, lane > 0 && before >= slot)) same = __match_any_sync(0xffffffffu, slot);
-                    if (r[j] != ~0ull && lane == 31 - __clz(same)) {
-                        ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v[j]);
-                        oc[slot] = (int32_t)(r[j] >> 32);
-                    }
-                    __syncwarp();
+                for (int j = 0; j < 4; ++j) {
+                    const int64_t i = b + j * FILL_LARGE_THREADS + tid;
+                    int row = 0;
+#pragma unroll
+                    for (int step = TILE_ROWS / 2; step > 0; step >>= 1) row += i >= start[row + step] ? step : 0;
+                    if (i < end) ov[(int64_t)(slot[j] >> 3) * TILE_ELEMS + row * TILE_COLS + (slot[j] & 7)] = from_float<T>(v[j]);
                 }
+            }
+            continue;
+        }
+        const int64_t last = start[warp + 1];
+        for (int64_t b = start[warp]; b < last; b += 32 * FILL_AHEAD) {
+            uint64_t r[FILL_AHEAD];
+            float v[FILL_AHEAD];
+#pragma unroll
+            for (int j = 0; j < FILL_AHEAD; ++j) {
+                const int64_t i = b + j * 32 + lane;
+                r[j] = i < last ? __ldg(s.rec + i) : ~0ull;
+                v[j] = i < last ? __ldg(s.val + i) : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < FILL_AHEAD; ++j) {
+                const uint32_t slot = (uint32_t)r[j];                     // all ones in an empty entry, no slot is
+                const unsigned same = __match_any_sync(0xffffffffu, slot);
+                if (r[j] != ~0ull && lane == 31 - __clz(same))
+                    ov[(int64_t)(slot >> 3) * TILE_ELEMS + warp * TILE_COLS + (slot & 7)] = from_float<T>(v[j]);
+                __syncwarp();
             }
         }
     }
@@ -716,10 +768,8 @@ size_t grws_csr_to_bcsr_scratch_bytes(int64_t num_rows, int64_t nnz) {
     return carve(nullptr, nnz, num_rows).total;
 }
 
-__attribute__((visibility("default")))
-int grws_csr_to_bcsr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
-                           const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
-                           size_t scratch_bytes, void *stream) {
+static int csr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx, const float *values, int64_t nnz, bool unique,
+                     int64_t *window_offset, void *scratch, size_t scratch_bytes, void *stream) {
     GRWS_REQUIRE(num_rows >= 0 && nnz >= 0, "negative size");
     GRWS_REQUIRE(nnz < 0x7fffffffLL, "csr_to_bcsr handles fewer than 2^31 entries");
     const int64_t W = ceil_div(num_rows, TILE_ROWS);
@@ -728,8 +778,22 @@ int grws_csr_to_bcsr_count(int64_t num_rows, const int64_t *row_ptr, const int32
     GRWS_REQUIRE(nnz == 0 || (col_idx && values), "null CSR arrays");
     BuildScratch s = carve(scratch, nnz, num_rows);
     if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small: %zu < %zu", scratch_bytes, s.total);
-    const EntrySource src = {row_ptr, col_idx, values, num_rows, 0};
+    const EntrySource src = {row_ptr, col_idx, values, num_rows, 0, unique};
     return count_entries(s, src, W, nnz > SMALL_ENTRIES, window_offset, static_cast<cudaStream_t>(stream));
+}
+
+__attribute__((visibility("default")))
+int grws_csr_to_bcsr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
+                           const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
+                           size_t scratch_bytes, void *stream) {
+    return csr_count(num_rows, row_ptr, col_idx, values, nnz, false, window_offset, scratch, scratch_bytes, stream);
+}
+
+__attribute__((visibility("default")))
+int grws_csr_to_bcsr_count_unique(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
+                                  const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
+                                  size_t scratch_bytes, void *stream) {
+    return csr_count(num_rows, row_ptr, col_idx, values, nnz, true, window_offset, scratch, scratch_bytes, stream);
 }
 
 // The kernels only visit the entries that row_ptr covers, so a bound on their number needs nothing of its own.
@@ -751,7 +815,7 @@ int grws_block_build_count(const int32_t *local, const float *w, int64_t n_dst, 
     GRWS_REQUIRE(window_offset && scratch && (n_entries == 0 || (local && w)), "null pointer");
     BuildScratch s = carve(scratch, n_entries, n_dst);
     if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "block build scratch too small: %zu < %zu", scratch_bytes, s.total);
-    const EntrySource src = {nullptr, local, w, n_dst, fanout};
+    const EntrySource src = {nullptr, local, w, n_dst, fanout, false};
     return count_entries(s, src, W, lists_may_be_large(fanout), window_offset, static_cast<cudaStream_t>(stream));
 }
 

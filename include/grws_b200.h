@@ -195,6 +195,12 @@ int grws_csr_to_bcsr_count_bounded(int64_t num_rows, const int64_t *row_ptr, con
                                    int64_t *window_offset, void *scratch, size_t scratch_bytes,
                                    void *stream);
 
+/* The count phase for entries of which no two have the same row and column (the transposed entries of a
+ * BCSR matrix): the fill then need not keep their order.  nnz may be a bound, as above. */
+int grws_csr_to_bcsr_count_unique(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
+                                  const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
+                                  size_t scratch_bytes, void *stream);
+
 /* The count phase straight from a hop's fixed-stride neighbour lists (this, with
  * grws_csr_to_bcsr_fill, replaces build_col_to_val_map_kernel + recompress_sampled_bcsr_kernel,
  * core/include/sampling.cuh:471-579,707-773): row i has the entries local[i*fanout + j] >= 0

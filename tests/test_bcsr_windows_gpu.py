@@ -62,3 +62,21 @@ def test_blocks_from_lists(oracle, fanout):
     assert np.array_equal(cols[:T * 8].cpu().numpy(), want[1])
     assert np.array_equal(vals[:T * 128].float().cpu().numpy(), want[2])
     assert bool((cols[T * 8:] == -1).all()) and bool((vals[T * 128:] == 0).all())
+
+
+@pytest.mark.parametrize("order", ["ascending", "any"])
+@pytest.mark.parametrize("num_cols", [3000, 1_200_000])
+def test_large_windows_of_distinct_entries(oracle, num_cols, order):
+    """Entries that can be written in any order: rows in ascending order (recognised), or the caller's word."""
+    from graph_rws_b200 import core
+    rng = np.random.default_rng(num_cols)
+    rows = [0, 1, 700, 0, 2999, 2998, 5, 0, 0, 600, 13, 0, 0, 0, 0, 2000, 0, 0, 300, 400, 33, 0, 800]
+    cols = [rng.choice(num_cols, m, replace=False).astype(np.int32) for m in rows]
+    if order == "ascending":
+        cols = [np.sort(c) for c in cols]
+    rp, ci = np.concatenate([[0], np.cumsum(rows)]).astype(np.int64), np.concatenate(cols)
+    v = rng.standard_normal(ci.size).astype(np.float32)
+    dev = torch.device("cuda")
+    wo, c, x = core.csr_to_bcsr(len(rows), *(torch.from_numpy(a).to(dev) for a in (rp, ci, v)), unique=order == "any")
+    for got, want in zip((wo, c, x), oracle.csr_to_bcsr(len(rows), rp, ci, v)):
+        assert np.array_equal(got.cpu().numpy(), want)
