@@ -1,5 +1,5 @@
 """Windows of the device builder at the edges of its two ways (a warp's sort of up to 512 entries, the
-column bitmap above), with duplicates and unsorted rows: bit-exact against the CPU checker."""
+column bitmap above), with duplicates and unsorted rows: bit-exact against the oracle."""
 import numpy as np
 import pytest
 import torch
