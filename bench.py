@@ -913,7 +913,7 @@ def secondary_sampled(args, torch, scale=1.0, steps=10):
            "roofline": {"bound": "hbm", "kernel": "sampling + dedup + block build (all hops of a step)", "achieved": achieved,
                         "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                         "algorithmic_bytes": sb, "launch_ms": samp_ms, "traffic": None,
-                        "note": "about 20 small kernels per hop: launch- and latency-bound, not bandwidth-bound"}}
+                        "note": "about 10 small kernels per hop: launch- and latency-bound, not bandwidth-bound"}}
     del model, opt, topo
     torch.cuda.empty_cache()
     return out
