@@ -542,10 +542,11 @@ transpose_entries_kernel(int64_t W, const int64_t *__restrict__ window_offset, c
                          int32_t *__restrict__ out_col, float *__restrict__ out_val, bool vec) {
     const int lane = threadIdx.x & 31;
     const int64_t n_warps = (int64_t)gridDim.x * TRANSPOSE_WARPS, me = (int64_t)blockIdx.x * TRANSPOSE_WARPS + (threadIdx.x >> 5);
-    const int64_t T0 = __ldg(window_offset + W);
-    int64_t share = (T0 + n_warps - 1) / n_warps;
+    // a range of the windows of a larger matrix, over that matrix's arrays, does not start at tile 0
+    const int64_t T_first = __ldg(window_offset), T0 = __ldg(window_offset + W);
+    int64_t share = (T0 - T_first + n_warps - 1) / n_warps;
     share = (share + TRANSPOSE_AHEAD - 1) / TRANSPOSE_AHEAD * TRANSPOSE_AHEAD;
-    const int64_t t0 = me * share, t1 = t0 + share < T0 ? t0 + share : T0;
+    const int64_t t0 = T_first + me * share, t1 = t0 + share < T0 ? t0 + share : T0;
     if (t0 >= t1) return;
     int64_t w = warp_count_ends_le(window_offset, W, t0, lane);      // the window that holds tile t0
     int64_t end = __ldg(window_offset + w + 1);
