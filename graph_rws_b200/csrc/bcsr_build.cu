@@ -401,12 +401,12 @@ fill_windows_kernel(int64_t W, int64_t num_rows, int64_t num_tiles, const BuildS
                 for (int i = 0; i < GROUP * TILE_COLS / 32; ++i) cb[i * 32 + lane] = -1;
                 __syncwarp();
                 while (p < end) {
-                    const int q = p + lane;
-                    const uint64_t r = q < end ? __ldg(s.rec + q) : ~0ull;
-                    const float v = q < end ? __ldg(s.val + q) : 0.f;
+                    const bool live = lane_has_entry(p, lane, end);
+                    const uint64_t r = live ? __ldg(s.rec + p + lane) : ~0ull;
+                    const float v = live ? __ldg(s.val + p + lane) : 0.f;
                     const uint32_t info = (uint32_t)r;
                     const int slot = (int)(info >> 5) - g * TILE_COLS;
-                    const bool in = q < end && slot < GROUP * TILE_COLS;
+                    const bool in = live && slot < GROUP * TILE_COLS;
                     if (in && !(info & 1u)) {
                         tb[(slot >> 3) * TILE_ELEMS + ((info >> 1) & (TILE_ROWS - 1)) * TILE_COLS + (slot & 7)] = from_float<T>(v);
                         cb[slot] = (int32_t)(r >> 32);

@@ -44,6 +44,10 @@ inline int fail(int status, const char *fmt, ...) {
 
 inline size_t dtype_bytes(int dt) { return dt == GRWS_F32 ? 4 : 2; }
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Does entry p + lane lie in [p, end)?  p + lane itself may be past the largest int.
+__host__ __device__ __forceinline__ bool lane_has_entry(int p, int lane, int end) { return lane < end - p; }
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------------------------
