@@ -269,15 +269,22 @@ def relabel_columns(cols, node_ids):
     return out
 
 
-def sanitize_columns(cols, values, num_cols):
-    """In place: ids of -1 or ``num_cols`` and more become 0, their column of the 16x8 tile zero."""
-    if not (cols.is_cuda and values.device == cols.device and cols.dtype == torch.int32 and values.dtype in _DT
-            and cols.is_contiguous() and values.is_contiguous()):
+def sanitize_columns(cols, values, num_cols, tile_rows=16, tile_cols=8):
+    """In place: ids of -1 or ``num_cols`` and more become 0, their column of the tile zero."""
+    # the kernel takes what it is told: whatever it does not cover, or autograd has a say in, goes through the
+    # tensor operations, which also refuse arrays that do not belong together
+    native = (cols.is_cuda and values.device == cols.device and cols.dtype == torch.int32 and values.dtype in _DT
+              and cols.is_contiguous() and values.is_contiguous() and (tile_rows, tile_cols) == (16, 8)
+              and cols.numel() % 8 == 0 and values.numel() == cols.numel() * 16
+              and not (values.requires_grad and torch.is_grad_enabled())
+              and (torch.is_inference_mode_enabled() or not (cols.is_inference() or values.is_inference())))
+    if not native:
         bad = (cols == -1) | (cols >= num_cols)
         cols.masked_fill_(bad, 0)
-        values.view(-1, 16, 8).masked_fill_(bad.view(-1, 1, 8), 0.0)
+        values.view(-1, tile_rows, tile_cols).masked_fill_(bad.view(-1, 1, tile_cols), 0.0)
         return
     _native.check(_native.lib().grws_sanitize_columns(_ptr(cols), _ptr(values), _DT[values.dtype], cols.numel() // 8, int(num_cols),
                                                       _stream(cols.device)))
-    torch.autograd.graph.increment_version(cols)          # what is cached for the old contents goes
-    torch.autograd.graph.increment_version(values)
+    for t in (cols, values):                                  # what is cached for the old contents goes
+        if not t.is_inference():
+            torch.autograd.graph.increment_version(t)

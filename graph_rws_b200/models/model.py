@@ -84,7 +84,7 @@ class GCN_BCSR(nn.Module):
         state = (g.original_col_indices.data_ptr(), g.values_condensed.data_ptr())
         if shared is not None and shared.get(key) == state:
             return
-        core.sanitize_columns(g.original_col_indices, g.values_condensed, num_src)
+        core.sanitize_columns(g.original_col_indices, g.values_condensed, num_src, g.tile_rows, g.tile_cols)
         if shared is not None:
             shared[key] = state
 
