@@ -67,6 +67,7 @@ SIGNATURES = {
                                          c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "grws_gather_rows_sharded": (c_i32, [c_vp, c_i32, c_i64, c_i64, c_i64, c_vp, c_i64, c_vp, c_vp]),
     "grws_relabel_columns": (c_i32, [c_vp, c_i64, c_vp, c_i64, c_vp, c_vp]),
+    "grws_relabel_columns_checked": (c_i32, [c_vp, c_i64, c_vp, c_i64, c_vp, c_vp, c_vp]),
     "grws_sanitize_columns": (c_i32, [c_vp, c_vp, c_i32, c_i64, c_i64, c_vp]),
     "grws_reindex_bcsr": (c_i32, [c_vp, c_vp, c_i32, c_vp, c_i64, c_i64, c_i32, c_i32, c_vp, c_vp]),
 }

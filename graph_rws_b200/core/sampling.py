@@ -259,13 +259,16 @@ def reindex_bcsr(col_indices, values_condensed, active_windows, tile_rows=16, ti
 
 
 def relabel_columns(cols, node_ids):
-    """``node_ids[cols]`` for the non-negative ids of ``cols`` (int32), the others as they are."""
+    """``node_ids[cols]`` for the non-negative ids of ``cols`` (int32), the others as they are.  An id past
+    ``node_ids`` stops the program at the next synchronisation, as indexing with it does."""
     if not (cols.is_cuda and cols.dtype == node_ids.dtype == torch.int32 and node_ids.device == cols.device):
         return torch.where(cols >= 0, node_ids[cols.clamp(min=0).long()], cols)
     cols, node_ids = cols.contiguous(), node_ids.contiguous()
     out = torch.empty_like(cols)
-    _native.check(_native.lib().grws_relabel_columns(_ptr(cols), cols.numel(), _ptr(node_ids), node_ids.numel(), _ptr(out),
-                                                     _stream(cols.device)))
+    ok = torch.empty(1, dtype=torch.int32, device=cols.device)
+    _native.check(_native.lib().grws_relabel_columns_checked(_ptr(cols), cols.numel(), _ptr(node_ids), node_ids.numel(), _ptr(out),
+                                                             _ptr(ok), _stream(cols.device)))
+    torch._assert_async(ok)
     return out
 
 

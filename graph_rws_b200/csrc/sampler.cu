@@ -287,12 +287,14 @@ __global__ void reindex_kernel(const int32_t *__restrict__ in_cols, T *__restric
     }
 }
 
-// column ids through a table: out[i] = map[cols[i]], negative ids as they are (an id past the table: -1)
+// column ids through a table: out[i] = map[cols[i]], negative ids as they are (an id past the table: -1, and *ok
+// becomes 0)
 __global__ void relabel_columns_kernel(const int32_t *__restrict__ cols, int64_t n, const int32_t *__restrict__ map, int64_t n_map,
-                                       int32_t *__restrict__ out) {
+                                       int32_t *__restrict__ out, int32_t *__restrict__ ok) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int32_t c = cols[i];
+    if (c >= n_map && ok) *ok = 0;
     out[i] = c < 0 ? c : c < n_map ? __ldg(map + c) : -1;
 }
 
@@ -637,14 +639,27 @@ int grws_reindex_bcsr(const int32_t *in_cols, void *values, int val_dtype, const
     return GRWS_OK;
 }
 
-__attribute__((visibility("default")))
-int grws_relabel_columns(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map, int32_t *out, void *stream) {
+static int relabel_columns(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map, int32_t *out, int32_t *ok, void *stream) {
     GRWS_REQUIRE(n >= 0 && n_map >= 0, "negative size");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (ok) GRWS_CUDA_TRY(cudaMemsetAsync(ok, 1, sizeof(*ok), st));
     if (n == 0) return GRWS_OK;
     GRWS_REQUIRE(cols && out && (n_map == 0 || map), "null pointer");
-    relabel_columns_kernel<<<nblocks(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(cols, n, map, n_map, out);
+    relabel_columns_kernel<<<nblocks(n, 256), 256, 0, st>>>(cols, n, map, n_map, out, ok);
     GRWS_CUDA_TRY(cudaGetLastError());
     return GRWS_OK;
+}
+
+__attribute__((visibility("default")))
+int grws_relabel_columns(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map, int32_t *out, void *stream) {
+    return relabel_columns(cols, n, map, n_map, out, nullptr, stream);
+}
+
+__attribute__((visibility("default")))
+int grws_relabel_columns_checked(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map, int32_t *out, int32_t *ok,
+                                 void *stream) {
+    GRWS_REQUIRE(ok, "null pointer");
+    return relabel_columns(cols, n, map, n_map, out, ok, stream);
 }
 
 __attribute__((visibility("default")))

@@ -339,11 +339,14 @@ int grws_block_compact(const int32_t *local, const float *w, int64_t n_dst, int 
 /* ------------------------------------------------------------------------------------------
  * Column ids of a block for the first layer (models/model.py:127-143 of the reference edits them with
  * tensor operations).  relabel: out[i] = map[cols[i]], negative ids as they are, -1 for an id past the map
- * (a block's local ids become global ones); sanitize, in place: ids of -1 or num_cols and more become
+ * (a block's local ids become global ones); relabel_checked also sets *ok to 0 where there was such an id,
+ * else to another value; sanitize, in place: ids of -1 or num_cols and more become
  * id 0 with zero values in their column of the tile.
  * ------------------------------------------------------------------------------------------ */
 int grws_relabel_columns(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map, int32_t *out,
                          void *stream);
+int grws_relabel_columns_checked(const int32_t *cols, int64_t n, const int32_t *map, int64_t n_map,
+                                 int32_t *out, int32_t *ok, void *stream);
 int grws_sanitize_columns(int32_t *cols, void *vals, int val_dtype, int64_t num_tiles, int64_t num_cols,
                           void *stream);
 

@@ -49,3 +49,14 @@ def test_other_tiles():
     c, v = _arrays(tile=(8, 4))
     core.sanitize_columns(c, v, 7, 8, 4)
     assert torch.equal(v.view(5, 8, 4).sum(1).flatten().cpu(), 8.0 * torch.tensor([0] + [1] * 7 + [0] * 12))
+
+
+@pytest.mark.parametrize("top,fine", [(49, True), (50, False), (2 ** 31 - 1, False)])
+def test_ids_past_the_table(monkeypatch, top, fine):
+    """Such an id stops the program; here the condition is taken down instead of being asserted."""
+    from graph_rws_b200 import core
+    seen = []
+    monkeypatch.setattr(torch, "_assert_async", lambda ok, *a: seen.append(bool(ok)))
+    cols = torch.tensor([3, -1, top, 0], dtype=torch.int32, device="cuda")
+    core.relabel_columns(cols, torch.arange(100, 150, dtype=torch.int32, device="cuda"))
+    assert seen == [fine]
