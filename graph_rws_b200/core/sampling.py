@@ -148,7 +148,7 @@ def sample_layers_sizes(num_seeds, fanouts, pad_to=0):
 
 
 def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_SEED, values_dtype=torch.float32,
-                        pad_to=0, seed_dev=None, want_counts=False):
+                        pad_to=0, seed_dev=None, want_counts=False, num_cols=None):
     """All hops of a mini-batch in ONE library call and without any size read-back.
 
     Same sampling, dedup and block layout as ``sample_layers_csr``; what differs is the sizing: every
@@ -157,6 +157,8 @@ def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_S
     shapes of a step depend only on (number of seeds, fanouts) and recur from step to step.  The
     call queues about ten kernels per hop on the current stream and returns; ctypes releases the
     interpreter lock for its duration, so a sampling thread does not hold up the training thread.
+    ``num_cols``: the number of columns where there are more of them than rows (the last hop may then
+    name nodes that have no row).  Ids past both are allowed there too, but are put in order more slowly.
 
     Returns one [window_offset, cols, vals, dst_nodes, src_nodes] list per hop (fanouts in the order
     given) and, with ``want_counts``, an int64 [hops, 4] device tensor {source nodes, sampled edges,
@@ -175,7 +177,7 @@ def sample_layers_fused(row_ptr, col_idx, values, seeds, fanouts, seed=DEFAULT_S
     vals_all = torch.empty(sum(t * 128 for t in tiles) + 8, dtype=values_dtype, device=dev)
     wo_sizes = [(n + 15) // 16 + 1 for n in n_dst]
     wo_all = torch.empty(sum(-(-n // 32) * 32 for n in wo_sizes) + 4 * L, dtype=torch.int64, device=dev)
-    num_nodes = row_ptr.numel() - 1
+    num_nodes = min(max(row_ptr.numel() - 1, int(num_cols or 0)), 2 ** 31 - 2)      # an id is an int32
     scratch = _scratch(lib.grws_sample_layers_sized_scratch_bytes(num_nodes, seeds.numel(), fan, L, int(pad_to)), dev)
     srcs, cols, vals, wos = [], [], [], []
     o32 = ov = ow = 0

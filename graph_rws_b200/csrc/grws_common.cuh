@@ -50,6 +50,35 @@ __host__ __device__ __forceinline__ bool lane_has_entry(int p, int lane, int end
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// Ascending bitonic sort of n keys in shared memory (n a power of two) by all threads of a block.  Steps of a stride of at
+// most 32 keep to the 64 keys of a warp's 32 pairs, so two of them in a row need no barrier of the block.
+__device__ __forceinline__ void block_sort(uint32_t *key, int n) {
+    __syncthreads();
+    for (int size = 2; size <= n; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int i = threadIdx.x; i < n / 2; i += blockDim.x) {
+                const int a = 2 * i - (i & (stride - 1)), b = a + stride;
+                const uint32_t x = key[a], y = key[b];
+                if ((x > y) == ((a & size) == 0)) { key[a] = y; key[b] = x; }
+            }
+            const int next = stride > 1 ? stride >> 1 : size;
+            if (stride > 32 || next > 32) __syncthreads(); else __syncwarp();
+        }
+    }
+    __syncthreads();
+}
+
+// number of keys below x in the ascending array key[0, n)
+template <typename Key>
+__device__ __forceinline__ int lower_bound(const Key *key, int n, Key x) {
+    int lo = 0;
+    while (n > 0) {
+        const int half = n >> 1;
+        if (key[lo + half] < x) { lo += half + 1; n -= half + 1; } else n = half;
+    }
+    return lo;
+}
+
 // ---------------------------------------------------------------------------------------------
 // work partition of one SpMM over the global tile array
 //

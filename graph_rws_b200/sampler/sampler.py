@@ -106,7 +106,7 @@ class BCSRSampler:
         if self.fused:
             hops = core.sample_layers_fused(row_ptr, col_idx, values, seed_nodes, reversed_fanouts,
                                             seed=self.seed + self.step, values_dtype=block_dtype,
-                                            pad_to=self.pad_to, seed_dev=seed_dev)
+                                            pad_to=self.pad_to, seed_dev=seed_dev, num_cols=getattr(g, 'num_cols', None))
             timing_list = []
         else:
             hops, timing_list = core.sample_layers_csr(row_ptr, col_idx, values, seed_nodes, reversed_fanouts,

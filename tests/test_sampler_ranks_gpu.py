@@ -44,3 +44,43 @@ def test_batch_table(oracle, n, num_cols, fanouts):
         assert np.array_equal(cols[:cols_r.size], cols_r) and (cols[cols_r.size:] == -1).all()
         assert np.array_equal(vals[:vals_r.size], vals_r) and (vals[vals_r.size:] == 0).all()
         dst = src
+
+
+@pytest.mark.parametrize("n,num_cols,fanout", [
+    (700, 2 ** 31 - 1, 12),         # one short run of ids past the node count
+    (3000, 2_000_000, 12),          # three runs, merged in two groups
+    (9000, 9_000_000, 30),          # some twenty runs in groups of eight, the last group short
+    (40000, 50_000, 32),            # most of the 10 k such ids are met many times
+])
+@pytest.mark.parametrize("told", [False, True])
+def test_many_ids_past_the_node_count(oracle, n, num_cols, fanout, told):
+    from graph_rws_b200 import core
+    csr = _csr(n, 2 * fanout, num_cols, n)
+    seeds = np.random.default_rng(2).permutation(n).astype(np.int32)
+    wo, cols, vals, _, src = (t.cpu().numpy() for t in core.sample_layers_fused(
+        *(torch.from_numpy(a).cuda() for a in (*csr, seeds)), [fanout], seed=9, num_cols=num_cols if told else None)[0])
+    nbr, w, _ = oracle.sample_hop(*csr, seeds, fanout, 9, 0)
+    src_r, wo_r, cols_r, vals_r = oracle.build_block(seeds, nbr, w)
+    assert np.array_equal(src[:src_r.size], src_r) and (src[src_r.size:] == -1).all()
+    assert np.array_equal(wo, wo_r)
+    assert np.array_equal(cols[:cols_r.size], cols_r) and np.array_equal(vals[:vals_r.size], vals_r)
+
+
+def test_ids_past_the_node_count_cost_no_more_than_a_sort():
+    """120 k such ids in one hop: near the time of a square graph's hop (a scan of their list for each took forty
+    times as long)."""
+    from graph_rws_b200 import core
+    times = []
+    for num_cols in (20000, 5_000_000):
+        csr = [torch.from_numpy(a).cuda() for a in _csr(20000, 60, num_cols, 5)]
+        seeds = torch.randperm(20000, generator=torch.Generator().manual_seed(1))[:8192].int().cuda()
+        taken = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            core.sample_layers_fused(*csr, seeds, [15], seed=9)
+            b.record()
+            b.synchronize()
+            taken.append(a.elapsed_time(b))
+        times.append(min(taken))
+    assert times[1] < 6 * times[0]
