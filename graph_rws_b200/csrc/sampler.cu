@@ -750,16 +750,32 @@ struct LayersScratch {
     float *w;
     void *dedup, *build;
     size_t dedup_bytes, build_bytes, total;
-    // with a known node count (instead of `dedup`)
+    // where the new nodes are ranked by a bitmap (instead of `dedup`)
+    bool bitmap;
     int32_t *keys, *vals, *counters;
     uint32_t *bits;                                  // [num_hops * words]
     HopRank rank;
     int64_t slots;
 };
 
+// The bitmap is cleared, counted and walked as a whole in every hop, so it is for graphs that are not too large for the
+// batch: a sort of a few thousand new ids is one launch, one of more takes 40 us and up.  A mini-batch with the bitmap /
+// with sorts, us, by its seeds and fan-outs (list slots of all hops: 1.3 k, 31 k, 39 k, 1.1 M):
+//   nodes      37, 5-5     256, 10-10   37, 15-10-5   1024, 15-10-5
+//   2.4 M     148 / 170     160 / 237     204 / 335      312 / 543
+//    20 M     179 / 165     175 / 227     226 / 326      308 / 490
+//    50 M     238 / 163     204 / 220     270 / 327      342 / 476
+//   111 M     357 / 172     262 / 224     357 / 326      440 / 472
+static bool ranks_by_bitmap(int64_t num_nodes, const int64_t *n_dst, const int *fanouts, int num_hops) {
+    int64_t slots = 0;
+    for (int h = 0; h < num_hops; ++h) slots += n_dst[h] * fanouts[h];
+    return num_nodes > 0 && ceil_div(num_nodes, 32) <= 450000 + 60 * (slots < 40000 ? slots : 40000) + slots;
+}
+
 static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const int *fanouts, int num_hops, int64_t pad_to, LayersScratch *out) {
     int64_t n_dst[16], n_src[16];
     if (int st = grws_sample_layers_sizes(num_seeds, fanouts, num_hops, pad_to, n_dst, n_src, nullptr)) return st;
+    const bool bitmap = ranks_by_bitmap(num_nodes, n_dst, fanouts, num_hops);
     size_t entries = 1, rows = 1, dedup = 0, build = 0;
     int64_t nodes = 1;
     for (int h = 0; h < num_hops; ++h) {
@@ -767,7 +783,7 @@ static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const 
         if (e > entries) entries = e;
         if ((size_t)n_dst[h] > rows) rows = (size_t)n_dst[h];
         if (n_src[h] > nodes) nodes = n_src[h];
-        const size_t d = num_nodes > 0 ? 0 : carve_dedup(nullptr, n_dst[h], fanouts[h]).total;
+        const size_t d = bitmap ? 0 : carve_dedup(nullptr, n_dst[h], fanouts[h]).total;
         const size_t b = grws_csr_to_bcsr_scratch_bytes(n_dst[h], (int64_t)e);
         if (d > dedup) dedup = d;
         if (b > build) build = b;
@@ -783,7 +799,8 @@ static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const 
     out->build = take(build);
     out->dedup_bytes = dedup;
     out->build_bytes = build;
-    if (num_nodes > 0) {
+    out->bitmap = bitmap;
+    if (bitmap) {
         int64_t slots = 64;
         while (slots < 2 * nodes + 16) slots <<= 1;  // every node of the batch: the last source list holds them all
         const int64_t words = ceil_div(num_nodes, 32);
@@ -844,7 +861,7 @@ int grws_sample_layers_sized(const int64_t *row_ptr, int64_t num_nodes, const in
     const int32_t *dst = seeds;
     const uint32_t table_mask = (uint32_t)(s.slots - 1);
     const unsigned rank_blocks = (unsigned)ceil_div(s.rank.words, RANK_THREADS);
-    if (num_nodes > 0 && num_seeds > 0) {
+    if (s.bitmap && num_seeds > 0) {
         const unsigned nb = nblocks(s.slots / 4, 256);
         layers_init_kernel<<<nb > 1184 ? 1184 : nb, 256, 0, st>>>(s.keys, s.vals, s.slots, s.bits, s.rank.words * num_hops, s.counters, 4 * num_hops);
         insert_seeds_kernel<<<nblocks(num_seeds, 256), 256, 0, st>>>(seeds, num_seeds, s.keys, s.vals, table_mask);
@@ -863,7 +880,7 @@ int grws_sample_layers_sized(const int64_t *row_ptr, int64_t num_nodes, const in
         if (int e = launch_sample_hop(row_ptr, col_idx, values, dst, nd, (int)f, seed, seed_dev, (uint32_t)h, s.nbr, s.w, s.cnt, st)) return e;
         // 2. source list = frontier ++ ascending new nodes ++ -1 padding; local id of every neighbour
         const int32_t *n_new;
-        if (num_nodes > 0) {
+        if (s.bitmap) {
             HopRank r = s.rank;
             r.bits = s.bits + s.rank.words * h;
             r.counters = s.counters + 4 * h;

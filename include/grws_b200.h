@@ -386,7 +386,8 @@ int grws_sample_layers(const int64_t *row_ptr, const int32_t *col_idx, const flo
 
 /* The same for a graph of num_nodes nodes (or columns, where it has more of them): the new nodes of a
  * hop are put in order through a bitmap of the node ids instead of a sort, with one hash table for
- * all hops.  num_nodes = 0: not known, as above.  Ids of num_nodes or more stay allowed where the
+ * all hops, unless the graph is so large for the batch that the sorts cost less.  num_nodes = 0: not known,
+ * as above.  Ids of num_nodes or more stay allowed where the
  * call above allows them, as neighbours in the last hop: they are sorted in runs and merged, which takes
  * longer than the bitmap and, from half a million of them in a hop on, longer than the call above. */
 size_t grws_sample_layers_sized_scratch_bytes(int64_t num_nodes, int64_t num_seeds, const int *fanouts,

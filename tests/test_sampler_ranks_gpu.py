@@ -84,3 +84,27 @@ def test_ids_past_the_node_count_cost_no_more_than_a_sort():
             taken.append(a.elapsed_time(b))
         times.append(min(taken))
     assert times[1] < 6 * times[0]
+
+
+@pytest.mark.parametrize("nodes,bitmap", [(1, True), (14_400_000, True), (17_000_000, False), (2 ** 31 - 2, False)])
+def test_small_batches_of_large_graphs_are_sorted(oracle, nodes, bitmap):
+    """37 seeds, fan-out 5-5 (1,295 list slots): the bitmap up to 450,000 words and 61 for every slot, sorts above; the
+    scratch tells which, the result does not."""
+    import ctypes
+    from graph_rws_b200 import core
+    from graph_rws_b200.core import _native
+    fan = (ctypes.c_int * 2)(5, 5)
+    lib = _native.lib()
+    sized = lib.grws_sample_layers_sized_scratch_bytes(nodes, 37, fan, 2, 0)
+    assert (sized != lib.grws_sample_layers_scratch_bytes(37, fan, 2, 0)) == bitmap
+    csr = _csr(500, 12, 500, 3)
+    seeds = np.arange(0, 74, 2, dtype=np.int32)
+    got = core.sample_layers_fused(*(torch.from_numpy(a).cuda() for a in (*csr, seeds)), [5, 5], seed=9, num_cols=nodes)
+    dst = seeds
+    for h in range(2):
+        wo, cols, vals, _, src = (t.cpu().numpy() for t in got[h])
+        nbr, w, _ = oracle.sample_hop(*csr, dst, 5, 9, h)
+        src_r, wo_r, cols_r, vals_r = oracle.build_block(dst, nbr, w)
+        assert np.array_equal(src[:src_r.size], src_r) and (src[src_r.size:] == -1).all() and np.array_equal(wo, wo_r)
+        assert np.array_equal(cols[:cols_r.size], cols_r) and np.array_equal(vals[:vals_r.size], vals_r)
+        dst = src
