@@ -788,7 +788,8 @@ static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const 
         if (d > dedup) dedup = d;
         if (b > build) build = b;
     }
-    char *p = static_cast<char *>(base);
+    // the buffers start on 256-byte boundaries (the table is cleared in 16-byte pieces), wherever the caller's scratch does
+    char *p = reinterpret_cast<char *>(up256(reinterpret_cast<uintptr_t>(base)));
     size_t off = 0;
     auto take = [&](size_t bytes) { char *q = p ? p + off : nullptr; off += up256(bytes); return (void *)q; };
     out->nbr = (int32_t *)take(entries * 4);
@@ -816,7 +817,7 @@ static int carve_layers(void *base, int64_t num_nodes, int64_t num_seeds, const 
         out->rank.over = (int32_t *)take(entries * 4);
         out->rank.merged = (int32_t *)take(entries * 4);
     }
-    out->total = off;
+    out->total = off + 255;
     return GRWS_OK;
 }
 

@@ -108,3 +108,16 @@ def test_small_batches_of_large_graphs_are_sorted(oracle, nodes, bitmap):
         assert np.array_equal(src[:src_r.size], src_r) and (src[src_r.size:] == -1).all() and np.array_equal(wo, wo_r)
         assert np.array_equal(cols[:cols_r.size], cols_r) and np.array_equal(vals[:vals_r.size], vals_r)
         dst = src
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8, 255])
+@pytest.mark.parametrize("nodes", [300, 2 ** 31 - 2])
+def test_scratch_may_start_anywhere(monkeypatch, offset, nodes):
+    from graph_rws_b200 import core
+    from graph_rws_b200.core import sampling
+    args = [torch.from_numpy(a).cuda() for a in (*_csr(300, 12, 300, 3), np.arange(0, 74, 2, dtype=np.int32))]
+    want = core.sample_layers_fused(*args, [5, 4], seed=9, num_cols=nodes)
+    monkeypatch.setattr(sampling, "_scratch", lambda n, dev: torch.empty(n + 256, dtype=torch.uint8, device=dev)[offset:offset + n])
+    got = core.sample_layers_fused(*args, [5, 4], seed=9, num_cols=nodes)
+    for a, b in zip(got, want):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
