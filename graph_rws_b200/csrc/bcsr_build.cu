@@ -779,6 +779,10 @@ static int csr_count(int64_t num_rows, const int64_t *row_ptr, const int32_t *co
     GRWS_REQUIRE(nnz == 0 || (col_idx && values), "null CSR arrays");
     BuildScratch s = carve(scratch, nnz, num_rows);
     if (scratch_bytes < s.total) return fail(GRWS_ERR_SCRATCH, "csr_to_bcsr scratch too small: %zu < %zu", scratch_bytes, s.total);
+    if (nnz == 0) {                            // row_ptr is not read then: it may be as short as the caller's entries
+        GRWS_CUDA_TRY(cudaMemsetAsync(window_offset, 0, (size_t)(W + 1) * 8, static_cast<cudaStream_t>(stream)));
+        return GRWS_OK;
+    }
     const EntrySource src = {row_ptr, col_idx, values, num_rows, 0, unique};
     return count_entries(s, src, W, nnz > SMALL_ENTRIES, window_offset, static_cast<cudaStream_t>(stream));
 }

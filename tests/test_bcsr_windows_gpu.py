@@ -80,3 +80,15 @@ def test_large_windows_of_distinct_entries(oracle, num_cols, order):
     wo, c, x = core.csr_to_bcsr(len(rows), *(torch.from_numpy(a).to(dev) for a in (rp, ci, v)), unique=order == "any")
     for got, want in zip((wo, c, x), oracle.csr_to_bcsr(len(rows), rp, ci, v)):
         assert np.array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("rows", [0, 16, 40])
+@pytest.mark.parametrize("exact", [True, False])
+def test_no_entries(rows, exact):
+    """Without entries the row pointers are not read (here there is only one)."""
+    from graph_rws_b200 import core
+    none = torch.empty(0, device="cuda")
+    wo, cols, vals = core.csr_to_bcsr(rows, torch.zeros(1, dtype=torch.int64, device="cuda"), none.int(), none, exact=exact)
+    windows = (rows + 15) // 16
+    assert wo.tolist() == [0] * (windows + 1)
+    assert cols.tolist() == [-1] * (0 if exact else windows * 8) and not vals.any()
