@@ -4,7 +4,8 @@
 //   The entries of a 16-row window are one contiguous range of the CSR arrays, so a window is
 //   built by itself: its entries are ordered by (column, row), equal columns become one column
 //   slot, slot / 8 is the tile, and the last duplicate of a (row, column) pair wins
-//   (convert_wrapper.cpp:174).  No pass goes over the whole graph more than once per phase.
+//   (convert_wrapper.cpp:174).  A window of up to 512 entries is read once per phase, a larger one four
+//   to six times by its CTA when it is counted, whatever its columns span.
 //
 //   BCSR -> transposed CSR: extracts the non-zero entries of the tiles as (column, row, value)
 //   so that the transposed adjacency can be built once, cached and multiplied with the forward
@@ -19,15 +20,19 @@
 namespace grws {
 
 // A window of up to SMALL_ENTRIES entries is sorted by one warp in registers (16 keys a lane); a larger
-// one is ranked by a CTA through a bitmap of its columns, whose cost does not grow with log(entries).
-// 512 covers every block of a sampled step up to fan-out 32 and all but the hub windows of a power-law
-// graph; 32 keys a lane would spill.
+// one is ranked by a CTA through a bitmap of its columns, or by a sort where they span more than that.
+// 512 covers every block of a sampled step up to fan-out 32, and all but the hub windows of a power-law
+// graph of up to about 25 entries a row; 32 keys a lane would spill.
 constexpr int SMALL_ENTRIES = 512;
 constexpr int COUNT_WARPS = 8;
 constexpr int LARGE_THREADS = 1024;
-constexpr int BITMAP_WORDS = 16384;                // 524,288 columns per round of a large window
+constexpr int BITMAP_WORDS = 16384;                // columns of a bitmap / 32
+constexpr uint32_t BITMAP_COLS = BITMAP_WORDS * 32u;
+constexpr int SORT_ENTRIES = 8 * LARGE_THREADS;    // entries of a large window that are sorted at a time where its columns span more than a bitmap
+constexpr int PART_BINS = 2048;                    // column ranges that such a window's entries are divided into first, if they are more
 constexpr int LARGE_SMEM = BITMAP_WORDS * 4 + BITMAP_WORDS / 2 * 4;   // bits + one prefix per word pair: two CTAs per SM
-constexpr int LARGE_PLAIN = 1 << 30;               // flag in BuildScratch::large (there are fewer than 2^28 windows)
+constexpr int LARGE_PLAIN = 1 << 30;               // flags in BuildScratch::large (there are fewer than 2^28 windows)
+constexpr int LARGE_WIDE = 1 << 29, LARGE_MIXED = 1 << 28;      // within count_large_kernel: still to be numbered; in no order
 constexpr int FILL_WARPS = 8;
 constexpr int FILL_BYTES = 4096;                   // tiles a warp assembles in shared memory at a time
 constexpr int FILL_LARGE_THREADS = 512;            // one warp per row of a window
@@ -56,14 +61,15 @@ struct EntrySource {
 //   rec, of a window of at most SMALL_ENTRIES entries (ordered by column slot):
 //         column << 32 | slot << 5 | row in window << 1 | 1 if the entry is not written (an empty list
 //         slot, or an earlier duplicate of the same row and column)
-//   rec, of a larger window (in the order of the source): column << 32 | slot, all ones for an empty slot
+//   rec, of a larger window (in the order of the source): column << 32 | slot, all ones for an empty slot or an entry
+//         that a later one of the same place takes the place of
 struct BuildScratch {
     uint64_t *rec;
     float *val;             // value of the entry rec describes
     int32_t *row_start;     // [num_rows + 1]
     int64_t *tiles;         // [W+1] tiles per window, shifted by one
-    int32_t *large;         // [1 + W] number of large windows, then their ids in no fixed order (bit 30: its entries are
-                            // all distinct, so they can be written in any order)
+    int32_t *large;         // [1 + W] number of large windows, then their ids in no fixed order (bit 30: no two of its
+                            // entries have one place, so they can be written in any order)
     int32_t *columns;       // [W] distinct columns of the large window listed at that place
     int32_t *ucol;          // column of every slot of a large window, from its first entry's place on
     void *cub_tmp;
@@ -241,117 +247,410 @@ __device__ __forceinline__ uint32_t block_reduce(uint32_t v, bool take_min, uint
     return take_min ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
 }
 
-// Large windows, one CTA each: the columns that occur are marked in a bitmap in shared memory, a prefix sum
-// of its bit counts gives every column its slot.  A window whose columns span more than the bitmap takes
-// further rounds, each starting at the smallest column not yet numbered.
-__global__ void __launch_bounds__(LARGE_THREADS, 2)
-count_large_kernel(const EntrySource src, BuildScratch s) {
-    extern __shared__ uint32_t smem[];
-    __shared__ uint32_t warp_part[LARGE_THREADS / 32];
-    __shared__ int out_of_order;
-    uint32_t *bits = smem, *prefix = smem + BITMAP_WORDS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_large = s.large[0];
-    for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
-        const int64_t w = s.large[1 + q], first = src.row_start(w * TILE_ROWS), m = src.row_start((w + 1) * TILE_ROWS) - first;
-        const int32_t *col = src.col + first;
-        uint32_t lo = 0xffffffffu, hi = 0;
-        bool any = false;
-        for (int64_t i = tid; i < m; i += LARGE_THREADS) {
-            const int32_t c = __ldg(col + i);
-            if (src.empty(c)) continue;
-            any = true;
-            lo = min(lo, (uint32_t)c);
-            hi = max(hi, (uint32_t)c);
-        }
-        any = __syncthreads_or(any);
-        lo = block_reduce(lo, true, warp_part);
-        hi = block_reduce(hi, false, warp_part);
-        uint32_t total = 0;
-        bool more = any;
-        while (more) {
-            const uint64_t left = (uint64_t)hi - lo + 1;
-            const uint32_t span = left < BITMAP_WORDS * 32ull ? (uint32_t)left : BITMAP_WORDS * 32u;
-            const int pairs = (int)((span + 63) / 64);
-            for (int i = tid; i < pairs; i += LARGE_THREADS) reinterpret_cast<uint2 *>(bits)[i] = make_uint2(0u, 0u);
+// exclusive prefix sum over a block of LARGE_THREADS
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warp_part, uint32_t *all) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    __syncthreads();                                                  // the previous use of warp_part is over
+    if (lane == 31) warp_part[warp] = incl;
+    __syncthreads();
+    const uint32_t part = warp_part[lane];
+    const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? part : 0u);
+    *all = __reduce_add_sync(0xffffffffu, part);
+    return ahead + incl - v;
+}
+
+// Ascending bitonic sort of LARGE_THREADS * E keys by a CTA; key i is k[i % E] of thread i / E.  Every warp sorts its own in
+// registers; a merge of sorted halves compares a key with its mirror image first, so that all of them ascend, and
+// only the exchanges between warps go through shared memory (15, in two buffers by turns: one barrier each).
+template <int E>
+__device__ __forceinline__ void block_sort(uint32_t (&k)[E], uint32_t *buf) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    warp_sort<E, uint32_t>(k, lane);
+    int turn = 0;
+    for (int warps = 2; warps <= LARGE_THREADS / 32; warps <<= 1) {
+        for (int d = warps * 32 - 1; d >= 32; d = d == warps * 32 - 1 ? warps * 8 : d >> 1) {
+            uint32_t *b = buf + turn * LARGE_THREADS * E;
+            const bool mirror = d == warps * 32 - 1, low = (tid & (mirror ? warps * 16 : d)) == 0;
+            turn ^= 1;
+#pragma unroll
+            for (int e = 0; e < E; ++e) b[e * LARGE_THREADS + tid] = k[e];
             __syncthreads();
-            uint32_t next = 0xffffffffu;
-            bool beyond = false;
-            for (int64_t i = tid; i < m; i += LARGE_THREADS) {
-                const int32_t c = __ldg(col + i);
-                if (src.empty(c) || (uint32_t)c < lo) continue;
-                const uint32_t x = (uint32_t)c - lo;
-                if (x < span) {
-                    atomicOr(bits + (x >> 5), 1u << (x & 31));
-                } else {
-                    beyond = true;
-                    next = min(next, (uint32_t)c);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint32_t o = b[(mirror ? E - 1 - e : e) * LARGE_THREADS + (tid ^ d)];
+                k[e] = low ? min(k[e], o) : max(k[e], o);
+            }
+        }
+#pragma unroll
+        for (int stride = 16 * E; stride > 0; stride >>= 1) {
+            if (stride >= E) {
+                const bool low = (lane & (stride / E)) == 0;
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, k[e], stride / E);
+                    k[e] = low ? min(k[e], o) : max(k[e], o);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    if (e & stride) continue;
+                    const uint32_t x = k[e], y = k[e + stride];
+                    k[e] = min(x, y);
+                    k[e + stride] = max(x, y);
                 }
             }
-            more = __syncthreads_or(beyond);
-            // exclusive prefix of the bit counts, one word pair at a time per thread
-            const int each = (pairs + LARGE_THREADS - 1) / LARGE_THREADS, p0 = tid * each, p1 = min(pairs, p0 + each);
-            uint32_t sum = 0;
-            for (int i = p0; i < p1; ++i) {
-                const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
-                sum += __popc(v.x) + __popc(v.y);
+        }
+    }
+    __syncthreads();                                                  // the buffers are free again
+}
+
+// Entries of one large window, in the order of the source
+struct LargeWindow {
+    EntrySource src;
+    const int32_t *col;
+    int64_t m;
+    uint64_t *rec;
+    int32_t *ucol;
+    __device__ __forceinline__ LargeWindow(const EntrySource &from, const BuildScratch &s, int64_t w) : src(from) {
+        const int64_t first = src.row_start(w * TILE_ROWS);
+        m = src.row_start((w + 1) * TILE_ROWS) - first;
+        col = src.col + first;
+        rec = s.rec + first;
+        ucol = s.ucol + first;
+    }
+};
+extern __shared__ uint32_t large_smem[];             // LARGE_SMEM bytes
+__device__ __forceinline__ uint32_t *large_part() {  // one word per warp
+    __shared__ uint32_t part[LARGE_THREADS / 32];
+    return part;
+}
+
+// Numbers the columns of the m entries `entry` gives, which lie in [from, to], by a bitmap in shared memory (one per round:
+// a range wider than the bitmap takes several, each from the smallest column not yet numbered) and a prefix sum of
+// its bit counts.  Writes the records and the columns of the slots from `total` on; returns their end.
+// ONE: the range is no wider than the bitmap.
+template <bool ONE, typename Entry>
+__device__ __forceinline__ uint32_t number_by_bitmap(const LargeWindow &win, int64_t m, const Entry &entry, uint32_t from, uint32_t to, uint32_t total) {
+    const int tid = threadIdx.x;
+    uint32_t *bits = large_smem, *prefix = large_smem + BITMAP_WORDS;
+    bool more = true;
+    while (more) {
+        const uint64_t left = (uint64_t)to - from + 1;
+        const uint32_t span = left < BITMAP_COLS ? (uint32_t)left : BITMAP_COLS;
+        const int pairs = (int)((span + 63) / 64);
+        for (int i = tid; i < pairs; i += LARGE_THREADS) reinterpret_cast<uint2 *>(bits)[i] = make_uint2(0u, 0u);
+        __syncthreads();
+        uint32_t next = 0xffffffffu;
+        bool beyond = false;
+        for (int64_t k = tid; k < m; k += LARGE_THREADS) {
+            const int32_t c = __ldg(win.col + entry(k));
+            if (win.src.empty(c) || (!ONE && (uint32_t)c < from)) continue;
+            const uint32_t x = (uint32_t)c - from;
+            if (ONE || x < span) {
+                atomicOr(bits + (x >> 5), 1u << (x & 31));
+            } else {
+                beyond = true;
+                next = min(next, (uint32_t)c);
             }
-            uint32_t incl = sum;
+        }
+        if (ONE) { more = false; __syncthreads(); } else more = __syncthreads_or(beyond);
+        // exclusive prefix of the bit counts, one word pair at a time per thread
+        const int each = (pairs + LARGE_THREADS - 1) / LARGE_THREADS, p0 = tid * each, p1 = min(pairs, p0 + each);
+        uint32_t sum = 0, round;
+        for (int i = p0; i < p1; ++i) {
+            const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
+            sum += __popc(v.x) + __popc(v.y);
+        }
+        uint32_t at = total + block_exclusive(sum, large_part(), &round);
+        for (int i = p0; i < p1; ++i) {
+            const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
+            prefix[i] = at;
+            const uint32_t c0 = from + (uint32_t)i * 64;
+            for (uint32_t b = v.x; b; b &= b - 1) win.ucol[at++] = (int32_t)(c0 + __ffs(b) - 1);
+            for (uint32_t b = v.y; b; b &= b - 1) win.ucol[at++] = (int32_t)(c0 + 31 + __ffs(b));
+        }
+        __syncthreads();
+        for (int64_t k = tid; k < m; k += LARGE_THREADS) {
+            const int64_t i = entry(k);
+            const int32_t c = __ldg(win.col + i);
+            if (win.src.empty(c) || (!ONE && (uint32_t)c < from)) continue;
+            const uint32_t x = (uint32_t)c - from;
+            if (!ONE && x >= span) continue;
+            const uint2 v = reinterpret_cast<uint2 *>(bits)[x >> 6];
+            const uint32_t below = (1u << (x & 31)) - 1u;
+            const uint32_t slot = prefix[x >> 6] + (x & 32 ? __popc(v.x) + __popc(v.y & below) : __popc(v.x & below));
+            win.rec[i] = (uint64_t)(uint32_t)c << 32 | slot;
+        }
+        total += round;
+        if (more) from = block_reduce(next, true, large_part());
+        __syncthreads();                                              // bits and prefix are free again
+    }
+    return total;
+}
+
+// The same by a sort of at most LARGE_THREADS * E entries, whatever their columns span
+template <int E, typename Entry>
+__device__ __forceinline__ uint32_t number_by_sort(const LargeWindow &win, int m, const Entry &entry, uint32_t total) {
+    const int tid = threadIdx.x;
+    uint32_t k[E], real = 0, found;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += o;
-            }
-            if (lane == 31) warp_part[warp] = incl;
+    for (int e = 0; e < E; ++e) {
+        k[e] = 0xffffffffu;                                           // behind or beside the largest column
+        const int i = e * LARGE_THREADS + tid;
+        const int32_t c = i < m ? __ldg(win.col + entry(i)) : 0;
+        if (i < m && !win.src.empty(c)) { k[e] = (uint32_t)c; ++real; }
+    }
+    block_exclusive(real, large_part(), &real);
+    block_sort<E>(k, large_smem);
+    large_smem[tid] = k[E - 1];                                         // the last key of every thread
+    __syncthreads();
+    uint32_t before = tid ? large_smem[tid - 1] : 0u, heads = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = (uint32_t)(tid * E + e);
+        if (i < real && (i == 0 || k[e] != before)) heads |= 1u << e;
+        before = k[e];
+    }
+    uint32_t *distinct = large_smem + LARGE_THREADS * E, at = block_exclusive(__popc(heads), large_part(), &found);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (heads >> e & 1u) distinct[at++] = k[e];
+    __syncthreads();
+    for (int i = tid; i < (int)found; i += LARGE_THREADS) win.ucol[total + i] = (int32_t)distinct[i];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int j = e * LARGE_THREADS + tid;
+        if (j >= m) break;
+        const int64_t i = entry(j);
+        const int32_t c = __ldg(win.col + i);
+        if (!win.src.empty(c)) win.rec[i] = (uint64_t)(uint32_t)c << 32 | (total + (uint32_t)lower_bound(distinct, (int)found, (uint32_t)c));
+    }
+    __syncthreads();                                                  // the keys are free again
+    return total + found;
+}
+
+template <typename Entry>
+__device__ __forceinline__ uint32_t number_by_sort(const LargeWindow &win, int64_t m, const Entry &entry, uint32_t total) {
+    if (m <= LARGE_THREADS) return number_by_sort<1>(win, (int)m, entry, total);
+    if (m <= 2 * LARGE_THREADS) return number_by_sort<2>(win, (int)m, entry, total);
+    if (m <= 4 * LARGE_THREADS) return number_by_sort<4>(win, (int)m, entry, total);
+    return number_by_sort<8>(win, (int)m, entry, total);
+}
+
+// smallest and largest column of a large window; false: it has none
+__device__ __forceinline__ bool column_span(const LargeWindow &win, uint32_t *lo_out, uint32_t *hi_out) {
+    uint32_t lo = 0xffffffffu, hi = 0;
+    bool any = false;
+    for (int64_t i = threadIdx.x; i < win.m; i += LARGE_THREADS) {
+        const int32_t c = __ldg(win.col + i);
+        if (win.src.empty(c)) continue;
+        any = true;
+        lo = min(lo, (uint32_t)c);
+        hi = max(hi, (uint32_t)c);
+    }
+    any = __syncthreads_or(any);
+    *lo_out = block_reduce(lo, true, large_part());
+    *hi_out = block_reduce(hi, false, large_part());
+    return any;
+}
+
+// The values of a large window; true where its rows are in strictly ascending order, that is, where every place at which
+// the columns do not ascend lies between two rows
+__device__ __forceinline__ bool copy_values(const LargeWindow &win, int64_t w, const float *__restrict__ from, float *__restrict__ to) {
+    __shared__ int out_of_order;
+    const int tid = threadIdx.x;
+    if (tid == 0) out_of_order = 0;
+    __syncthreads();
+    int odd = 0;
+    for (int64_t i = tid; i < win.m; i += LARGE_THREADS) {
+        const int32_t c = __ldg(win.col + i);
+        if (win.src.empty(c)) win.rec[i] = ~0ull;
+        if (i + 1 < win.m && (uint32_t)c >= (uint32_t)__ldg(win.col + i + 1)) ++odd;
+        to[i] = __ldg(from + i);
+    }
+    if (tid > 0 && tid < TILE_ROWS) {
+        const int64_t first = win.src.row_start(w * TILE_ROWS);
+        const int64_t at = win.src.row_start(w * TILE_ROWS + tid) - first, before = win.src.row_start(w * TILE_ROWS + tid - 1) - first;
+        if (at > before && at < win.m && (uint32_t)__ldg(win.col + at - 1) >= (uint32_t)__ldg(win.col + at)) --odd;
+    }
+    if (odd) atomicAdd(&out_of_order, odd);
+    __syncthreads();
+    return out_of_order == 0;
+}
+
+// A large window whose columns span more than a few bitmaps is sorted in shared memory, so that its cost depends on its
+// entries and not on the number of columns.  (Further bitmap rounds cost less where they are few and the entries many:
+// with 4,800 entries a window 2.0 ms against 2.6 ms for two rounds, 2.5 ms each for three; with 14,400 entries 2.6 ms
+// against 3.8 ms for three, about even for ten.)  One of more than SORT_ENTRIES entries is divided by column ranges first
+// (`order` lists them by range; it lies where their values will be) and goes on range by range, each with the way
+// that takes it further.
+__device__ __forceinline__ uint32_t number_wide_window(const LargeWindow &win, uint32_t lo, uint32_t hi, int32_t *order) {
+    __shared__ uint32_t bin_end[PART_BINS];
+    const int tid = threadIdx.x;
+    auto all_entries = [](int64_t k) { return k; };
+    const uint32_t rounds = (hi - lo) / BITMAP_COLS + 1u;
+    if (rounds <= (win.m > SORT_ENTRIES ? 8u : win.m > 2 * LARGE_THREADS ? 2u : 0u))
+        return number_by_bitmap<false>(win, win.m, all_entries, lo, hi, 0u);
+    if (win.m <= SORT_ENTRIES) return number_by_sort(win, win.m, all_entries, 0u);
+    int shift = 0;
+    while ((hi - lo) >> shift >= (uint32_t)PART_BINS) ++shift;
+    const int bins = (int)((hi - lo) >> shift) + 1;
+    for (int i = tid; i < PART_BINS; i += LARGE_THREADS) bin_end[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int64_t i = tid; i < win.m; i += LARGE_THREADS) {
+        const int32_t c = __ldg(win.col + i);
+        if (!win.src.empty(c)) atomicAdd(bin_end + (((uint32_t)c - lo) >> shift), 1u);
+    }
+    __syncthreads();
+    static_assert(PART_BINS == 2 * LARGE_THREADS, "two bins a thread");
+    const uint32_t n0 = bin_end[2 * tid], n1 = bin_end[2 * tid + 1];
+    uint32_t all;
+    const uint32_t at = block_exclusive(n0 + n1, large_part(), &all);
+    bin_end[2 * tid] = at;
+    bin_end[2 * tid + 1] = at + n0;
+    __syncthreads();
+#pragma unroll 4
+    for (int64_t i = tid; i < win.m; i += LARGE_THREADS) {
+        const int32_t c = __ldg(win.col + i);
+        if (!win.src.empty(c)) order[atomicAdd(bin_end + (((uint32_t)c - lo) >> shift), 1u)] = (int32_t)i;
+    }
+    __syncthreads();                                                  // bin_end now holds where each bin ends
+    uint32_t total = 0;
+    for (int bin = 0; bin < bins;) {
+        const uint32_t k0 = bin ? bin_end[bin - 1] : 0u;
+        const int by_width = (int)(BITMAP_COLS >> shift);             // bins a bitmap takes
+        const int by_count = lower_bound(bin_end + bin, bins - bin, k0 + SORT_ENTRIES + 1u);       // bins a sort takes
+        const int next = min(bins, bin + max(1, max(by_width, by_count)));
+        const uint32_t from = lo + ((uint32_t)bin << shift), to = next < bins ? lo + ((uint32_t)next << shift) - 1u : hi;
+        const int64_t m = bin_end[next - 1] - k0;
+        const int32_t *mine = order + k0;
+        auto entry = [mine](int64_t k) { return (int64_t)mine[k]; };
+        bin = next;
+        if (m == 0) continue;
+        if (by_count > 0 && by_count >= by_width) total = number_by_sort(win, m, entry, total);
+        else total = number_by_bitmap<false>(win, m, entry, from, to, total);
+    }
+    return total;
+}
+
+// Takes the records of all but the last entry of every (row, column slot) of a large window away.  A row is walked from its
+// end, a chunk at a time, over a bitmap of the slots that have been met; entries of one slot in one chunk are told
+// apart by a list of such slots.
+__device__ __forceinline__ void drop_superseded(const LargeWindow &win, int64_t w, uint32_t total) {
+    __shared__ int n_twice;
+    uint32_t *bits = large_smem, *twice = large_smem + BITMAP_WORDS, *last = twice + LARGE_THREADS;
+    const int tid = threadIdx.x;
+    const int64_t first = win.src.row_start(w * TILE_ROWS);
+    for (uint32_t base = 0; base < total; base += BITMAP_COLS) {
+        const uint32_t span = min(total - base, BITMAP_COLS);
+        for (int r = 0; r < TILE_ROWS; ++r) {
+            const int64_t i0 = win.src.row_start(w * TILE_ROWS + r) - first, i1 = win.src.row_start(w * TILE_ROWS + r + 1) - first;
+            for (int i = tid; i < (int)((span + 31) / 32); i += LARGE_THREADS) bits[i] = 0u;
+            if (tid == 0) n_twice = 0;
             __syncthreads();
-            const uint32_t part = warp_part[lane];
-            const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? part : 0u);
-            const uint32_t round = __reduce_add_sync(0xffffffffu, part);
-            uint32_t at = total + ahead + incl - sum;
-            for (int i = p0; i < p1; ++i) {
-                const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
-                prefix[i] = at;
-                const uint32_t c0 = lo + (uint32_t)i * 64;
-                for (uint32_t b = v.x; b; b &= b - 1) s.ucol[first + at++] = (int32_t)(c0 + __ffs(b) - 1);
-                for (uint32_t b = v.y; b; b &= b - 1) s.ucol[first + at++] = (int32_t)(c0 + 31 + __ffs(b));
+            for (int64_t end = i1; end > i0; end -= LARGE_THREADS) {
+                const int64_t i = end - LARGE_THREADS + tid;
+                const uint32_t x = i >= i0 ? (uint32_t)win.rec[i] - base : 0u, bit = 1u << (x & 31);
+                const bool in = i >= i0 && x < span && (uint32_t)win.rec[i] != 0xffffffffu;
+                const bool met = in && (bits[x >> 5] & bit) != 0;
+                __syncthreads();
+                bool lost = false;
+                if (in && !met && (atomicOr(bits + (x >> 5), bit) & bit) != 0) {
+                    lost = true;
+                    const int j = atomicAdd(&n_twice, 1);
+                    twice[j] = x;
+                    last[j] = 0u;
+                }
+                if (met) win.rec[i] = ~0ull;
+                if (!__syncthreads_or(lost)) continue;
+                const int n = n_twice;
+                for (int j = 0; j < n; ++j)
+                    if (in && !met && twice[j] == x) atomicMax(last + j, (uint32_t)tid + 1u);
+                __syncthreads();
+                for (int j = 0; j < n; ++j)
+                    if (in && !met && twice[j] == x && last[j] != (uint32_t)tid + 1u) win.rec[i] = ~0ull;
+                if (tid == 0) n_twice = 0;
+                __syncthreads();
             }
-            __syncthreads();
-            for (int64_t i = tid; i < m; i += LARGE_THREADS) {
-                const int32_t c = __ldg(col + i);
-                if (src.empty(c) || (uint32_t)c < lo) continue;
-                const uint32_t x = (uint32_t)c - lo;
-                if (x >= span) continue;
-                const uint2 v = reinterpret_cast<uint2 *>(bits)[x >> 6];
-                const uint32_t below = (1u << (x & 31)) - 1u;
-                const uint32_t slot = prefix[x >> 6] + (x & 32 ? __popc(v.x) + __popc(v.y & below) : __popc(v.x & below));
-                s.rec[first + i] = (uint64_t)(uint32_t)c << 32 | slot;
-            }
-            total += round;
-            if (more) lo = block_reduce(next, true, warp_part);
-            __syncthreads();                                          // bits and prefix are free again
+            __syncthreads();                                          // the row's bits are free again
         }
-        // values; and are the rows in strictly ascending order, that is: does every place where the columns do not
-        // ascend lie between two rows
-        if (tid == 0) out_of_order = 0;
-        __syncthreads();
-        int odd = 0;
-        for (int64_t i = tid; i < m; i += LARGE_THREADS) {
-            const int32_t c = __ldg(col + i);
-            if (src.empty(c)) s.rec[first + i] = ~0ull;
-            if (i + 1 < m && (uint32_t)c >= (uint32_t)__ldg(col + i + 1)) ++odd;
-            s.val[first + i] = __ldg(src.val + first + i);
+    }
+}
+
+// The windows that a CTA of count_large_kernel has left for later: those with columns further apart than a bitmap reaches
+// are numbered, and entries in no order are rid of duplicates where they are many (a hub's row written in order keeps
+// one warp busy for all of it).  A loop of its own: in one with the usual windows it cost those a quarter of their speed.
+// Builds, ms, with a bitmap round for every 524,288 columns / like this / with one radix sort of all entries:
+//   2.4 M rows of 52 entries, 2.4 M columns           33.2 / 10.9 / 14.9
+//   1 M rows of 40 entries, 100 M columns            357   /  3.9 /  4.9
+//   100 k rows of 300 entries, 600 k columns           2.0 /  2.2 /  3.6
+//   1 M rows of 12 and 500 of 100 k, 100 M columns    41.6 /  8.5 /  7.2   (4.0 where the rows ascend)
+//   16 rows of 1 M and nothing else, 100 M columns   111   / 15.0 /  3.9   (one CTA per hub: 132 of 148 SMs are idle)
+//   the same, 400 k columns, in no order              12.3 /  4.7 /  3.9
+__device__ __forceinline__ void count_left_windows(const EntrySource &src, const BuildScratch &s) {
+    const int n_large = s.large[0];
+    for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
+        const int32_t id = s.large[1 + q];
+        if (!(id & (LARGE_WIDE | LARGE_MIXED))) continue;
+        const int64_t w = id & ~(LARGE_WIDE | LARGE_MIXED);
+        const LargeWindow win(src, s, w);
+        uint32_t total = (uint32_t)s.columns[q];
+        bool plain = false;
+        if (id & LARGE_WIDE) {
+            uint32_t lo, hi;
+            column_span(win, &lo, &hi);
+            float *val = s.val + (win.rec - s.rec);
+            total = number_wide_window(win, lo, hi, reinterpret_cast<int32_t *>(val));
+            const bool ordered = copy_values(win, w, src.val + (win.col - src.col), val);
+            plain = src.row_ptr && (src.unique || ordered);
         }
-        if (tid > 0 && tid < TILE_ROWS) {
-            const int64_t at = src.row_start(w * TILE_ROWS + tid) - first, before = src.row_start(w * TILE_ROWS + tid - 1) - first;
-            if (at > before && at < m && (uint32_t)__ldg(col + at - 1) >= (uint32_t)__ldg(col + at)) --odd;
+        if (src.row_ptr && !plain && win.m > SORT_ENTRIES) {
+            drop_superseded(win, w, total);
+            plain = true;
         }
-        if (odd) atomicAdd(&out_of_order, odd);
-        __syncthreads();
-        if (tid == 0) {
+        __syncthreads();                                              // every thread has read the window's id and columns
+        if (threadIdx.x == 0) {
             s.tiles[w + 1] = ((int64_t)total + TILE_COLS - 1) / TILE_COLS;
             s.columns[q] = (int32_t)total;
-            s.large[1 + q] = (int32_t)w | (src.row_ptr && (src.unique || out_of_order == 0) ? LARGE_PLAIN : 0);
+            s.large[1 + q] = (int32_t)w | (plain ? LARGE_PLAIN : 0);
         }
+    }
+}
+
+// Large windows, one CTA each: every distinct column gets its slot, usually by one bitmap of all columns.  Bound by the
+// latency of its loads and barriers; two CTAs per SM (32 registers a thread) hide some of each other's.
+__global__ void __launch_bounds__(LARGE_THREADS, 2)
+count_large_kernel(const EntrySource src, const BuildScratch s) {
+    bool left = false;
+    const int n_large = s.large[0];
+    for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
+        const int64_t w = s.large[1 + q];
+        const LargeWindow win(src, s, w);
+        uint32_t lo, hi, total = 0;
+        int flags = LARGE_WIDE;
+        const bool any = column_span(win, &lo, &hi);
+        if (!any || hi - lo < BITMAP_COLS) {
+            if (any) total = number_by_bitmap<true>(win, win.m, [](int64_t k) { return k; }, lo, hi, 0u);
+            const bool ordered = copy_values(win, w, src.val + (win.col - src.col), s.val + (win.rec - s.rec));
+            flags = !src.row_ptr ? 0 : src.unique || ordered ? LARGE_PLAIN : win.m > SORT_ENTRIES ? LARGE_MIXED : 0;
+        }
+        left |= (flags & (LARGE_WIDE | LARGE_MIXED)) != 0;
+        if (threadIdx.x == 0) {
+            s.tiles[w + 1] = ((int64_t)total + TILE_COLS - 1) / TILE_COLS;
+            s.columns[q] = (int32_t)total;
+            s.large[1 + q] = (int32_t)w | flags;
+        }
+    }
+    if (left) {
+        __syncthreads();
+        count_left_windows(src, s);
     }
 }
 
@@ -431,9 +730,9 @@ fill_windows_kernel(int64_t W, int64_t num_rows, int64_t num_tiles, const BuildS
         store_piece(out_cols, i, make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu), vec);
 }
 
-// Large windows, one CTA each: column ids and empty tiles, then the entries are scattered.  Distinct entries go in any
-// order, all threads side by side; otherwise a warp per row keeps their order, so that the last of several entries of
-// one column is the one that stays.  Bound by the scattered stores of the CTA with the most entries: a hub's row has
+// Large windows, one CTA each: column ids and empty tiles, then the entries are scattered.  Where no two have one place
+// they go in any order, all threads side by side; otherwise a warp per row keeps their order, so that the last of
+// several entries of one column is the one that stays.  Bound by the scattered stores of the CTA with the most entries: a hub's row has
 // thousands and its 15 neighbours few, so a warp per row leaves 15 of 16 warps waiting.  A 169 k-node graph and its
 // transpose, fp32: 648 us built with a warp per row throughout, 548 us with distinct entries side by side.
 template <typename T>
@@ -467,7 +766,7 @@ fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restr
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int64_t i = b + j * FILL_LARGE_THREADS + tid;
-                    slot[j] = i < end ? (uint32_t)__ldg(s.rec + i) : 0u;
+                    slot[j] = i < end ? (uint32_t)__ldg(s.rec + i) : 0xffffffffu;
                     v[j] = i < end ? __ldg(s.val + i) : 0.f;
                 }
 #pragma unroll
@@ -476,7 +775,7 @@ fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restr
                     int row = 0;
 #pragma unroll
                     for (int step = TILE_ROWS / 2; step > 0; step >>= 1) row += i >= start[row + step] ? step : 0;
-                    if (i < end) ov[(int64_t)(slot[j] >> 3) * TILE_ELEMS + row * TILE_COLS + (slot[j] & 7)] = from_float<T>(v[j]);
+                    if (slot[j] != 0xffffffffu) ov[(int64_t)(slot[j] >> 3) * TILE_ELEMS + row * TILE_COLS + (slot[j] & 7)] = from_float<T>(v[j]);
                 }
             }
             continue;

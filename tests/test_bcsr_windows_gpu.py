@@ -92,3 +92,91 @@ def test_no_entries(rows, exact):
     windows = (rows + 15) // 16
     assert wo.tolist() == [0] * (windows + 1)
     assert cols.tolist() == [-1] * (0 if exact else windows * 8) and not vals.any()
+
+
+def _wide(kind, m, num_cols, rng):
+    if kind == "even":
+        return rng.integers(0, num_cols, m)
+    far = rng.integers(0, num_cols, m // 16)                   # most entries in a narrow band, the others anywhere
+    return rng.permutation(np.concatenate([num_cols // 3 + rng.integers(0, min(num_cols // 3, 700_000), m - far.size), far]))
+
+
+@pytest.mark.parametrize("kind", ["even", "band"])
+@pytest.mark.parametrize("num_cols", [524_287, 524_289, 600_000, 3_000_000, 7_000_000, 2 ** 31 - 1])
+def test_wide_windows(oracle, num_cols, kind):
+    """Large windows about as wide as a column bitmap and wider: a few rounds of bitmaps, one sort of up to 8,192 entries, or
+    divided by column ranges that are sorted or marked (of the band's ranges some hold more than a sort takes and
+    are wider than a bitmap)."""
+    from graph_rws_b200 import core
+    rng = np.random.default_rng(num_cols)
+    sizes = [513, 1024, 1025, 2048, 2049, 4100, 8191, 8192, 8193, 16_500, 200_000, 700]
+    counts = np.concatenate([np.bincount(rng.integers(0, 16, m), minlength=16) for m in sizes])
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    ci = np.concatenate([_wide(kind, m, num_cols, rng) for m in sizes]).astype(np.int32)
+    ci[rp[16 * 3]], ci[rp[16 * 3] + 1] = 0, num_cols - 1       # the whole span
+    v = rng.standard_normal(ci.size).astype(np.float32)
+    n = len(counts)
+    got = core.csr_to_bcsr(n, *(torch.from_numpy(a).cuda() for a in (rp, ci, v)))
+    for g, want in zip(got, oracle.csr_to_bcsr(n, rp, ci, v)):
+        assert np.array_equal(g.cpu().numpy(), want)
+
+
+def test_wide_blocks_from_lists(oracle):
+    """Lists whose local ids span more than a column bitmap, with empty slots."""
+    from graph_rws_b200 import core
+    rng = np.random.default_rng(8)
+    n, fanout = 2400, 256
+    rp = np.concatenate([[0], np.cumsum(rng.integers(200, 400, n))]).astype(np.int64)
+    ci = rng.integers(0, 2 ** 30, rp[-1]).astype(np.int32)
+    v = rng.standard_normal(rp[-1]).astype(np.float32)
+    seeds = rng.permutation(n).astype(np.int32)
+    wo, cols, vals, _, src = core.sample_layers_fused(*(torch.from_numpy(a).cuda() for a in (rp, ci, v, seeds)), [fanout], seed=3)[0]
+    nbr, w, _ = oracle.sample_hop(rp, ci, v, seeds, fanout, 3, 0)
+    src_r, wo_r, cols_r, vals_r = oracle.build_block(seeds, nbr, w)
+    assert cols_r.max() >= 524_288
+    assert np.array_equal(src[:src_r.size].cpu().numpy(), src_r) and np.array_equal(wo.cpu().numpy(), wo_r)
+    assert np.array_equal(cols[:cols_r.size].cpu().numpy(), cols_r) and np.array_equal(vals[:vals_r.size].cpu().numpy(), vals_r)
+
+
+def test_cost_does_not_grow_with_the_columns():
+    """Windows of 640 entries in 400 k and in 100 M columns: within a factor (each 524,288 columns used to cost every
+    window two more passes: a factor of 200)."""
+    from graph_rws_b200 import core
+    times = []
+    for num_cols in (400_000, 100_000_000):
+        g = torch.Generator(device="cuda").manual_seed(1)
+        rp = torch.arange(0, 100_001, device="cuda") * 40
+        ci = torch.randint(0, num_cols, (4_000_000,), generator=g, device="cuda", dtype=torch.int32)
+        v = torch.ones(4_000_000, device="cuda")
+        taken = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            core.csr_to_bcsr(100_000, rp, ci, v, exact=False)
+            b.record()
+            b.synchronize()
+            taken.append(a.elapsed_time(b))
+        times.append(min(taken))
+    assert times[1] < 8 * times[0]
+
+
+@pytest.mark.parametrize("twice", [None, "row", "other row"])
+@pytest.mark.parametrize("entries,num_cols", [(8193, 30_000), (20_000, 3_000_000), (600_000, 2_000_000), (30_000, 9_000_000)])
+def test_unordered_hub_row(oracle, entries, num_cols, twice):
+    """A long row in no order next to a short one: distinct entries (found out by more than a bitmap of slots in the
+    widest), a column twice in the row (the last one stays), or once in either row."""
+    from graph_rws_b200 import core
+    rng = np.random.default_rng(entries)
+    hub = rng.choice(num_cols, entries, replace=False).astype(np.int32)
+    short = rng.choice(num_cols, 300, replace=False).astype(np.int32)
+    if twice == "row":
+        hub[-1] = hub[entries // 3] = hub.max()                # the last slot, too
+    if twice == "other row":
+        short[7] = hub[-1]
+    rp = np.array([0] * 5 + [entries] * 4 + [entries + 300] * 11, dtype=np.int64)
+    ci = np.concatenate([hub, short])
+    v = rng.standard_normal(ci.size).astype(np.float32)
+    n = rp.size - 1
+    got = core.csr_to_bcsr(n, *(torch.from_numpy(a).cuda() for a in (rp, ci, v)))
+    for g, want in zip(got, oracle.csr_to_bcsr(n, rp, ci, v)):
+        assert np.array_equal(g.cpu().numpy(), want)
