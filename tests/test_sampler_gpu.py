@@ -152,7 +152,7 @@ def test_padded_hops_keep_the_real_part_identical(graph):
 
 @pytest.mark.parametrize("pad_to", [0, 512])
 def test_fused_all_hops_call_matches_replay(oracle, graph, pad_to):
-    """grws_sample_layers: every hop's source list, offsets, column ids and values equal the host
+    """All hops in one call: every hop's source list, offsets, column ids and values equal the host
     replay run on the same (padded) frontiers; buffers have the bound sizes and empty tails."""
     from graph_rws_b200 import core
     rp, ci, vv = _dev_csr(graph)

@@ -121,3 +121,27 @@ def test_scratch_may_start_anywhere(monkeypatch, offset, nodes):
     got = core.sample_layers_fused(*args, [5, 4], seed=9, num_cols=nodes)
     for a, b in zip(got, want):
         assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("pad_to", [0, 64])
+def test_entry_without_a_node_count(pad_to):
+    """grws_sample_layers, the call that is not told the number of nodes, gives the same hops and counts."""
+    import ctypes
+    from graph_rws_b200 import core
+    from graph_rws_b200.core import _native
+    lib = _native.lib()
+    rp, ci, vv = (torch.from_numpy(a).cuda() for a in _csr(3000, 12, 3000, 3))
+    seeds = torch.arange(0, 3000, 41, dtype=torch.int32, device="cuda")
+    fanouts = [5, 4]
+    want, counts = core.sample_layers_fused(rp, ci, vv, seeds, fanouts, seed=9, pad_to=pad_to, want_counts=True)
+    fan = (ctypes.c_int * 2)(*fanouts)
+    outs = [[torch.empty_like(t) for t in (hop[4], hop[0], hop[1], hop[2])] for hop in want]
+    got_counts = torch.empty_like(counts)
+    scratch = torch.empty(lib.grws_sample_layers_scratch_bytes(seeds.numel(), fan, 2, pad_to), dtype=torch.uint8, device="cuda")
+    arrays = [(ctypes.c_void_p * 2)(*[hop[i].data_ptr() for hop in outs]) for i in range(4)]
+    _native.check(lib.grws_sample_layers(rp.data_ptr(), ci.data_ptr(), vv.data_ptr(), seeds.data_ptr(), seeds.numel(), fan, 2, 9, 0, pad_to,
+                                         _native.F32, *arrays, got_counts.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                                         torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(got_counts, counts)
+    for hop, out in zip(want, outs):
+        assert all(torch.equal(a, b) for a, b in zip((hop[4], hop[0], hop[1], hop[2]), out))
