@@ -170,8 +170,9 @@ def csr_to_bcsr(num_rows, row_ptr, col_idx, values, tile_rows=16, tile_cols=8, v
     them walk ``window_offset``.  Per-step builders (sampled blocks, their transposes) use it.
     ``nnz_is_bound``: only the first ``row_ptr[num_rows]`` entries of ``col_idx`` / ``values`` exist,
     their length is a bound (the caller did not read the count back either); ``num_cols`` (with
-    ``nnz_is_bound``): every column id is below it.  ``unique``: no (row, column) pair occurs twice, so
-    the entries need not be kept in order."""
+    ``nnz_is_bound``): every column id is below it, which the builder can do without.  ``unique``: the
+    caller knows that no (row, column) pair occurs twice, so the entries need not be kept in order.  It
+    is not checked: of entries that do occur twice any one stays, not the same from call to call."""
     if tile_rows != 16 or tile_cols != 8:
         raise RuntimeError("Currently only supports tile 16x8")
     lib = _native.lib()

@@ -208,8 +208,10 @@ __device__ __forceinline__ int sort_window(const EntrySource &src, int64_t s, in
     return rank_window<E, unsigned long long>(k, src, s, m, ends, lane, rec, val);
 }
 
-// One warp per window.  Bound by instruction issue (the compare-exchange network: 36 steps of 8 keys a lane
-// for the usual window of up to 256 entries).  Against one radix sort of 64-bit (window, column, row) keys over all
+// One warp per window.  Bound by fetching its instructions and by the latency of its loads: warps stand 2.9 and 3.2 cycles an
+// instruction for them on a 169 k-node graph (10,584 windows), up to 9 and 2 on a sampled block, the pipes are 42 % and
+// less busy.  The sorting networks are unrolled for five sizes and two key widths, so that the time depends a
+// little on where the linker puts them (36 or 40 us for the three hops of a mini-batch).  Against one radix sort of 64-bit (window, column, row) keys over all
 // entries -- five to seven passes over keys and values, flags, two scans -- a mini-batch of 1,024 seeds and
 // fan-out 15-10-5 was sampled and built in 519 us instead of 769.
 __global__ void __launch_bounds__(COUNT_WARPS * 32, 3)
@@ -673,7 +675,8 @@ __device__ __forceinline__ void store_piece(T *p, int64_t i, uint4 v, bool vec) 
 }
 
 // One warp per window: the records are in slot order, so a group of consecutive tiles is a run of them; it is
-// assembled in shared memory and written once, in 16-byte pieces.  Bound by the bytes of the tiles.
+// assembled in shared memory and written once, in 16-byte pieces.  Bound by the latency of the records' loads (a warp
+// waits 13 cycles an instruction for them; DRAM is 19 % busy, 32 us for the 90 MB of a 169 k-node graph's fp16 tiles).
 // All threads then empty the tiles behind the last one (arrays sized by a bound).
 template <typename T>
 __global__ void __launch_bounds__(FILL_WARPS * 32)
@@ -732,9 +735,9 @@ fill_windows_kernel(int64_t W, int64_t num_rows, int64_t num_tiles, const BuildS
 
 // Large windows, one CTA each: column ids and empty tiles, then the entries are scattered.  Where no two have one place
 // they go in any order, all threads side by side; otherwise a warp per row keeps their order, so that the last of
-// several entries of one column is the one that stays.  Bound by the scattered stores of the CTA with the most entries: a hub's row has
-// thousands and its 15 neighbours few, so a warp per row leaves 15 of 16 warps waiting.  A 169 k-node graph and its
-// transpose, fp32: 648 us built with a warp per row throughout, 548 us with distinct entries side by side.
+// several entries of one column is the one that stays.  Bound by the CTA with the most entries and the latency of its loads:
+// a hub's row has thousands and its 15 neighbours few, so a warp per row leaves 15 of 16 warps waiting.  A 169 k-node
+// graph and its transpose, fp32: 648 us built with a warp per row throughout, 548 us with distinct entries side by side.
 template <typename T>
 __global__ void __launch_bounds__(FILL_LARGE_THREADS)
 fill_large_kernel(int64_t num_rows, const BuildScratch s, const int64_t *__restrict__ window_offset,
@@ -832,7 +835,7 @@ constexpr int TRANSPOSE_AHEAD = 4;     // tiles a warp has in flight
 // MODE 0 counts the non-zero entries per column, MODE 1 scatters them.  The tiles are shared out evenly over the
 // warps, whatever window they belong to: a hub's window has a hundred times the tiles of the others, and
 // with a CTA per window its chain of load, atomic and store was the kernel's time (169 k nodes, 315 k tiles of
-// fp32: counting 283 -> 51 us, scattering 383 -> 134 us; the tiles' bytes alone take 26 us).  vec: cols and vals start on
+// fp32: counting 283 -> 51 us, scattering 383 -> 90 us; the tiles' bytes alone take 26 us).  vec: cols and vals start on
 // 16-byte boundaries.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(TRANSPOSE_WARPS * 32)

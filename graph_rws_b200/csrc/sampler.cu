@@ -3,17 +3,19 @@
 // Replaces the sampling half of the reference's extension.  The reference samples per 16-row
 // window and keeps the top-K columns by edge weight (core/include/sampling.cuh:65-448, driven by
 // core/wrapper/sampling_wrapper.cu:58-438); it has no random generator.  Here a hop is
-//   1. sample_hop_kernel   one warp per frontier node: uniform sampling without replacement on a
-//                          counter-based Philox4x32-10 stream keyed by (seed, node, hop), so a
-//                          node's list does not depend on batch composition, launch shape or GPU
-//                          count (Floyd's subset algorithm; degree <= fanout takes every
-//                          neighbour in CSR order);
-//   2. dedup / reindex     a global-memory hash set of the destination nodes plus the sampled
-//                          neighbours: the source list of the hop is the destination nodes
-//                          followed by the new nodes in ascending id order (radix sort), and every
-//                          sampled edge gets the position of its endpoint in that list;
-//   3. compaction          the fixed-stride neighbour lists become a local CSR, which the
-//                          device BCSR builder (bcsr_build.cu) turns into the hop's block.
+//   1. sample_hop          a group of 4 to 32 lanes per frontier node (a warp above fan-out 32):
+//                          uniform sampling without replacement on a counter-based Philox4x32-10
+//                          stream keyed by (seed, node, hop), so a node's list does not depend on
+//                          batch composition, launch shape or GPU count (Floyd's subset algorithm;
+//                          degree <= fanout takes every neighbour in CSR order);
+//   2. dedup / reindex     a global-memory hash set of the nodes: the source list of the hop is the
+//                          destination nodes followed by the new nodes in ascending id order, and
+//                          every sampled edge gets the position of its endpoint in that list.  All
+//                          hops of a batch share one table, and a bitmap of the node ids gives the
+//                          order; single hops, graphs of unknown size and small batches of very
+//                          large graphs have a table per hop and a radix sort;
+//   3. block               the device BCSR builder (bcsr_build.cu) takes the fixed-stride lists as
+//                          they are, or, of a single hop, compacted to a local CSR.
 // reindex_and_prune_kernel (core/include/reindex.cuh:33-102) is kept as well, with the same
 // integer arithmetic, for graphs that carry the reference's window-level `active_windows`.
 #include <cub/cub.cuh>
@@ -301,7 +303,7 @@ __global__ void relabel_columns_kernel(const int32_t *__restrict__ cols, int64_t
 // Column slots that name no row of the operand (-1 padding, ids of num_cols or more) become slots of row 0 with
 // zero values.  Only such slots' values are written: eight neighbouring threads cover 16-byte rows of a tile.  (A
 // masked fill reads and writes all values: 45 us for the 33 MB of a sampled step's first block, and 60 us with the
-// comparisons around it; under 5 us like this.)
+// comparisons around it; 9.5 us like this, caches cold.)
 template <typename T>
 __global__ void sanitize_columns_kernel(int32_t *__restrict__ cols, T *__restrict__ vals, int64_t n, int64_t num_cols) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -196,7 +196,8 @@ int grws_csr_to_bcsr_count_bounded(int64_t num_rows, const int64_t *row_ptr, con
                                    void *stream);
 
 /* The count phase for entries of which no two have the same row and column (the transposed entries of a
- * BCSR matrix): the fill then need not keep their order.  nnz may be a bound, as above. */
+ * BCSR matrix): the fill then need not keep their order.  This is not checked: of several entries of one place
+ * any one stays, not the same from call to call.  nnz may be a bound, as above. */
 int grws_csr_to_bcsr_count_unique(int64_t num_rows, const int64_t *row_ptr, const int32_t *col_idx,
                                   const float *values, int64_t nnz, int64_t *window_offset, void *scratch,
                                   size_t scratch_bytes, void *stream);
