@@ -249,7 +249,8 @@ __device__ __forceinline__ uint32_t block_reduce(uint32_t v, bool take_min, uint
     return take_min ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
 }
 
-// exclusive prefix sum over a block of LARGE_THREADS
+// exclusive prefix sum over a block of LARGE_THREADS.  FREE: a barrier has passed since warp_part was read last.
+template <bool FREE = false>
 __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warp_part, uint32_t *all) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl = v;
@@ -258,7 +259,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warp_p
         const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += o;
     }
-    __syncthreads();                                                  // the previous use of warp_part is over
+    if (!FREE) __syncthreads();                                       // the previous use of warp_part is over
     if (lane == 31) warp_part[warp] = incl;
     __syncthreads();
     const uint32_t part = warp_part[lane];
@@ -328,15 +329,15 @@ struct LargeWindow {
     }
 };
 extern __shared__ uint32_t large_smem[];             // LARGE_SMEM bytes
-__device__ __forceinline__ uint32_t *large_part() {  // one word per warp
-    __shared__ uint32_t part[LARGE_THREADS / 32];
+__device__ __forceinline__ uint32_t *large_part() {  // two words per warp
+    __shared__ uint32_t part[2 * (LARGE_THREADS / 32)];
     return part;
 }
 
 // Numbers the columns of the m entries `entry` gives, which lie in [from, to], by a bitmap in shared memory (one per round:
 // a range wider than the bitmap takes several, each from the smallest column not yet numbered) and a prefix sum of
 // its bit counts.  Writes the records and the columns of the slots from `total` on; returns their end.
-// ONE: the range is no wider than the bitmap.
+// ONE: the range is no wider than the bitmap (and the caller passes a barrier before shared memory is used again).
 template <bool ONE, typename Entry>
 __device__ __forceinline__ uint32_t number_by_bitmap(const LargeWindow &win, int64_t m, const Entry &entry, uint32_t from, uint32_t to, uint32_t total) {
     const int tid = threadIdx.x;
@@ -369,7 +370,7 @@ __device__ __forceinline__ uint32_t number_by_bitmap(const LargeWindow &win, int
             const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
             sum += __popc(v.x) + __popc(v.y);
         }
-        uint32_t at = total + block_exclusive(sum, large_part(), &round);
+        uint32_t at = total + block_exclusive<true>(sum, large_part(), &round);
         for (int i = p0; i < p1; ++i) {
             const uint2 v = reinterpret_cast<uint2 *>(bits)[i];
             prefix[i] = at;
@@ -391,7 +392,7 @@ __device__ __forceinline__ uint32_t number_by_bitmap(const LargeWindow &win, int
         }
         total += round;
         if (more) from = block_reduce(next, true, large_part());
-        __syncthreads();                                              // bits and prefix are free again
+        if (!ONE) __syncthreads();                                    // bits and prefix are free again
     }
     return total;
 }
@@ -445,21 +446,27 @@ __device__ __forceinline__ uint32_t number_by_sort(const LargeWindow &win, int64
     return number_by_sort<8>(win, (int)m, entry, total);
 }
 
-// smallest and largest column of a large window; false: it has none
+// smallest and largest column of a large window; false: it has none.  One barrier: the caller passes another one before
+// it is called again or large_part is written.
 __device__ __forceinline__ bool column_span(const LargeWindow &win, uint32_t *lo_out, uint32_t *hi_out) {
-    uint32_t lo = 0xffffffffu, hi = 0;
-    bool any = false;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t *part = large_part(), lo = 0xffffffffu, hi = 0;
     for (int64_t i = threadIdx.x; i < win.m; i += LARGE_THREADS) {
         const int32_t c = __ldg(win.col + i);
         if (win.src.empty(c)) continue;
-        any = true;
         lo = min(lo, (uint32_t)c);
         hi = max(hi, (uint32_t)c);
     }
-    any = __syncthreads_or(any);
-    *lo_out = block_reduce(lo, true, large_part());
-    *hi_out = block_reduce(hi, false, large_part());
-    return any;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+        part[warp] = lo;
+        part[LARGE_THREADS / 32 + warp] = hi;
+    }
+    __syncthreads();
+    *lo_out = __reduce_min_sync(0xffffffffu, part[lane]);             // LARGE_THREADS / 32 == 32 warps
+    *hi_out = __reduce_max_sync(0xffffffffu, part[LARGE_THREADS / 32 + lane]);
+    return *lo_out <= *hi_out;
 }
 
 // The values of a large window; true where its rows are in strictly ascending order, that is, where every place at which
@@ -608,6 +615,7 @@ __device__ __forceinline__ void count_left_windows(const EntrySource &src, const
         if (id & LARGE_WIDE) {
             uint32_t lo, hi;
             column_span(win, &lo, &hi);
+            __syncthreads();
             float *val = s.val + (win.rec - s.rec);
             total = number_wide_window(win, lo, hi, reinterpret_cast<int32_t *>(val));
             const bool ordered = copy_values(win, w, src.val + (win.col - src.col), val);
@@ -638,7 +646,9 @@ count_large_kernel(const EntrySource src, const BuildScratch s) {
         uint32_t lo, hi, total = 0;
         int flags = LARGE_WIDE;
         const bool any = column_span(win, &lo, &hi);
-        if (!any || hi - lo < BITMAP_COLS) {
+        if (any && hi - lo >= BITMAP_COLS) {
+            __syncthreads();
+        } else {
             if (any) total = number_by_bitmap<true>(win, win.m, [](int64_t k) { return k; }, lo, hi, 0u);
             const bool ordered = copy_values(win, w, src.val + (win.col - src.col), s.val + (win.rec - s.rec));
             flags = !src.row_ptr ? 0 : src.unique || ordered ? LARGE_PLAIN : win.m > SORT_ENTRIES ? LARGE_MIXED : 0;
