@@ -494,17 +494,18 @@ __device__ __forceinline__ bool copy_values(const LargeWindow &win, int64_t w, c
 }
 
 // A large window whose columns span more than a few bitmaps is sorted in shared memory, so that its cost depends on its
-// entries and not on the number of columns.  (Further bitmap rounds cost less where they are few and the entries many:
-// with 4,800 entries a window 2.0 ms against 2.6 ms for two rounds, 2.5 ms each for three; with 14,400 entries 2.6 ms
-// against 3.8 ms for three, about even for ten.)  One of more than SORT_ENTRIES entries is divided by column ranges first
+// entries and not on the number of columns.  One of more than SORT_ENTRIES entries is divided by column ranges first
 // (`order` lists them by range; it lies where their values will be) and goes on range by range, each with the way
-// that takes it further.
+// that takes it further.  Further bitmap rounds cost less where they are few and the entries many.  Whole builds, ms, with
+// rounds / without: 4,800 entries a window, two rounds 2.2 / 2.6, three 2.5 / 2.5; 14,400 entries, six 3.5 / 3.7, eight
+// 3.9 / 3.7; 96,000 entries, eight 5.6 / 7.7, twelve 6.6 / 7.7.
 __device__ __forceinline__ uint32_t number_wide_window(const LargeWindow &win, uint32_t lo, uint32_t hi, int32_t *order) {
     __shared__ uint32_t bin_end[PART_BINS];
     const int tid = threadIdx.x;
     auto all_entries = [](int64_t k) { return k; };
     const uint32_t rounds = (hi - lo) / BITMAP_COLS + 1u;
-    if (rounds <= (win.m > SORT_ENTRIES ? 8u : win.m > 2 * LARGE_THREADS ? 2u : 0u))
+    const uint32_t few = win.m > SORT_ENTRIES ? 7u + (uint32_t)min(win.m >> 14, (int64_t)7) : win.m > 2 * LARGE_THREADS ? 2u : 0u;
+    if (rounds <= few)
         return number_by_bitmap<false>(win, win.m, all_entries, lo, hi, 0u);
     if (win.m <= SORT_ENTRIES) return number_by_sort(win, win.m, all_entries, 0u);
     int shift = 0;
@@ -597,12 +598,12 @@ __device__ __forceinline__ void drop_superseded(const LargeWindow &win, int64_t 
 // are numbered, and entries in no order are rid of duplicates where they are many (a hub's row written in order keeps
 // one warp busy for all of it).  A loop of its own: in one with the usual windows it cost those a quarter of their speed.
 // Builds, ms, with a bitmap round for every 524,288 columns / like this / with one radix sort of all entries:
-//   2.4 M rows of 52 entries, 2.4 M columns           33.2 / 10.9 / 14.9
-//   1 M rows of 40 entries, 100 M columns            357   /  3.9 /  4.9
+//   2.4 M rows of 52 entries, 2.4 M columns           33.2 / 10.4 / 14.9
+//   1 M rows of 40 entries, 100 M columns            357   /  3.8 /  4.9
 //   100 k rows of 300 entries, 600 k columns           2.0 /  2.2 /  3.6
-//   1 M rows of 12 and 500 of 100 k, 100 M columns    41.6 /  8.5 /  7.2   (4.0 where the rows ascend)
+//   1 M rows of 12 and 500 of 100 k, 100 M columns    41.6 /  8.3 /  7.2   (3.9 where the rows ascend)
 //   16 rows of 1 M and nothing else, 100 M columns   111   / 15.0 /  3.9   (one CTA per hub: 132 of 148 SMs are idle)
-//   the same, 400 k columns, in no order              12.3 /  4.7 /  3.9
+//   the same, 400 k columns, in no order              12.3 /  4.6 /  3.9
 __device__ __forceinline__ void count_left_windows(const EntrySource &src, const BuildScratch &s) {
     const int n_large = s.large[0];
     for (int q = blockIdx.x; q < n_large; q += gridDim.x) {
